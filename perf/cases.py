@@ -41,21 +41,21 @@ def _steps(name, sx, dx, rheology, steps, faults=1, gravity=False, afterslip=Fal
 def listed():
     return [
         # the smallest member shape of the ensembles, on its own: launches and host latency count
-        _steps("steps 64x64x64 maxwell", (64, 64, 64), 1.0, "maxwell", 20),
+        _steps("steps 64x64x64 maxwell", (64, 64, 64), 1.0, "maxwell", 40),
         # the linear Maxwell benchmark box
-        _steps("steps 128x128x128 maxwell", (128, 128, 128), 0.8, "maxwell", 20),
+        _steps("steps 128x128x128 maxwell", (128, 128, 128), 0.8, "maxwell", 40),
         # the headline benchmark: power law with an afterslip plane, adaptive time step
-        _steps("steps 256x256x128 afterslip", (256, 256, 128), 0.5, "powerlaw", 20, afterslip=True),
+        _steps("steps 256x256x128 afterslip", (256, 256, 128), 0.5, "powerlaw", 40, afterslip=True),
         # the large instance: three faults, gravity, a stress exponent that needs powf
-        dict(_steps("steps 512x512x256 gravity", (512, 512, 256), 0.4, "powerlaw", 6, faults=3, gravity=True),
+        dict(_steps("steps 512x512x256 gravity", (512, 512, 256), 0.4, "powerlaw", 16, faults=3, gravity=True),
              power=3.5),
         # the tutorials' 256^3 box, power law with gravity
-        _steps("steps 256x256x256 gravity", (256, 256, 256), 0.4, "powerlaw", 8, gravity=True),
+        _steps("steps 256x256x256 gravity", (256, 256, 256), 0.4, "powerlaw", 24, gravity=True),
         # transient (Burgers) rheology on top of the viscous one
-        _steps("steps 128x128x128 burgers", (128, 128, 128), 0.8, "burgers", 20),
+        _steps("steps 128x128x128 burgers", (128, 128, 128), 0.8, "burgers", 40),
         # ragged boxes, as chosen to fit a region rather than a power of two
-        _steps("steps 108x72x54 powerlaw", (108, 72, 54), 0.9, "powerlaw", 20),
-        _steps("steps 288x216x144 powerlaw", (288, 216, 144), 0.5, "powerlaw", 10, faults=2, gravity=True),
+        _steps("steps 108x72x54 powerlaw", (108, 72, 54), 0.9, "powerlaw", 40),
+        _steps("steps 288x216x144 powerlaw", (288, 216, 144), 0.5, "powerlaw", 20, faults=2, gravity=True),
         # one short solve from a deck to its fields (parameter sweeps, inversions)
         _steps("solve 96x96x64 maxwell", (96, 96, 64), 1.0, "maxwell", 10, kind="solve"),
         # an uneven ensemble: members of 64^3, 128^2 x 64, 128^3 and 192^2 x 96
@@ -93,7 +93,7 @@ def draw(rng):
         return {"kind": kind, "sx1": min(sx1, 256), "sx2": min(sx2, 256), "sx3": min(sx3, 144), "dx": dx,
                 "power": rng.choice([1.0, 3.0, 3.5]), "gravity": gravity}
     rheology = rng.choice(["maxwell", "powerlaw", "powerlaw", "burgers"])
-    c = _steps("", (sx1, sx2, sx3), dx, rheology, rng.randint(4, 6) if sx1 * sx2 * sx3 > 1 << 24 else rng.randint(5, 20),
+    c = _steps("", (sx1, sx2, sx3), dx, rheology, rng.randint(6, 12) if sx1 * sx2 * sx3 > 1 << 24 else rng.randint(8, 40),
                faults=rng.randint(1, 3), gravity=gravity, afterslip=rng.random() < 0.3, kind=kind)
     del c["name"]
     c["power"] = rng.choice([2.0, 3.0, 3.5])
