@@ -28,7 +28,7 @@ class RelaxError(RuntimeError):
 
 def build(verbose: bool = False):
     """Compiles the CUDA library for sm_100a (cross-compiles without a GPU)."""
-    out = subprocess.run(["make", "-s", "-C", os.path.join(HERE, "csrc")], capture_output=not verbose,
+    out = subprocess.run(["make", "-s", f"-j{os.cpu_count() or 1}", "-C", os.path.join(HERE, "csrc")], capture_output=not verbose,
                          text=True)
     if out.returncode != 0:
         raise RuntimeError("building librelax_b200.so failed:\n" + (out.stderr or "") + (out.stdout or ""))

@@ -7,6 +7,7 @@
 
 #include "common.cuh"
 #include "rfft.cuh"
+#include "spectral.cuh"
 
 namespace relax {
 // kernels and their argument types have internal linkage: each translation
@@ -64,53 +65,9 @@ __device__ __forceinline__ float tnorm6(float a, float b, float c, float d, floa
     return sqrtf((a * a + 2.f * b * b + 2.f * c * c + d * d + 2.f * e * e + f * f) * 0.5f);
 }
 
-// Programmatic dependent launch.  A kernel launched with the
-// programmatic-serialization attribute may be scheduled while the kernel
-// before it in the stream still runs; pdl_wait (griddepcontrol.wait) blocks
-// until that kernel has completed and its memory operations are visible, and
-// returns at once in a launch without the attribute.  pdl_trigger
-// (griddepcontrol.launch_dependents) lets the next kernel be scheduled once
-// every block of this one has issued it.  The step's streaming kernels call
-// both first thing, wait before trigger, so that at most the next kernel's
-// blocks are placed during a kernel's last wave, and none reads memory
-// before its wait.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_enter() { pdl_wait(); }
 
-__device__ __forceinline__ float4 ld4(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
-__device__ __forceinline__ float4 ldc4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
-__device__ __forceinline__ void st4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
-__device__ __forceinline__ float geti(const float4 &v, int j) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; }
 
-// 1/x by the hardware's approximate reciprocal (PTX rcp.approx.ftz.f32,
-// relative error about 2^-23; a subnormal x flushes to zero).  The x3
-// passes use it for the elastic response 1/|k|^2 and the Cerruti kernel
-// 1/((2 pi k3)^2 + beta^2), whose operands are positive and normal; it
-// takes the z pass from 69.6 to 66.5 us on the 256 x 256 x 128 box, with
-// a relative L2 difference of 4.5e-8 to the divided form.
-__device__ __forceinline__ float rcp_fast(float x)
-{
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
 
-// Derivatives along the periodic axes x1 and x2.  optimalfilter
-// (src/elastic3d.f90:846-907) takes the central difference
-// (w[i+1] - w[i-1]) / (2 dx) for sx <= 4 and sx >= 15, and the 7-point FIR
-// differentiator fir7 of src/kernel7.inc for 5 <= sx <= 14: sum over
-// l = 1..7 of (w[i+l] - w[i-l]) fir7(l) / dx, indexes periodic
-// (localstrain_ani, src/elastic3d.f90:1140-1178, and localdivergence_ani,
-// :1431-1470).  A Fir7 with n = 7 selects the filter, c[l-1] = fir7(l) / dx;
-// n = 0 the central difference.  Along x3, fir7 is selected for
-// 5 <= sx3/2 <= 14, but then every layer is a boundary layer of the filter
-// ((i3 > 7) and (i3 < sx3/2 - 6) is never true, stressupdate :975-976), so
-// the finite differences of localstrain_ani apply throughout.
-struct Fir7 {
-    int n;
-    float c[7];
-};
 
 // sum_l (w[(i2+l) % sx2] - w[(i2-l) % sx2]) c[l-1] at 4 consecutive points
 // of rows of pitch sx1 (w points at x1 of the row i2 = 0 of the plane)
@@ -1132,26 +1089,7 @@ __global__ void k_dgammadot0(Grid g, const relax_weakzone *zones, int nz, double
 // Output: spectrum planes [0, nin) and the traction plane sx3, scaled by
 // dx1 dx2 dx3 (dx1 dx2 for the traction), src/fourier.f90:195-199.
 // ------------------------------------------------------------------------
-enum { XIN_DIV = 0, XIN_REAL = 1 };
 
-struct XfArgs {
-    Grid g;
-    float2 *S;
-    FftPlan pm;              // complex length M = sx1/2
-    const float2 *tw1;       // exp(-2 pi i k / sx1)
-    int nin, rows;
-    int has_trac;            // blockIdx.y == nin is the traction plane
-    const float *m;          // XIN_DIV: 6 x nh moment
-    float k1, k2, k3, k3b;
-    Fir7 fx, fy;             // XIN_DIV: the x1, x2 differentiators (n = 7: fir7, k_xfwd only)
-    const float *in[3];      // XIN_REAL
-    size_t rp, pp;           // row / plane pitch (elements)
-    const float *tin[3];
-    size_t trp;
-    const float *tload;      // optional surface load added to t3 (sx1 x sx2)
-    float scale3, scale2;
-    const struct XfArgs *tab;   // batched launch: one entry per member (blockIdx.z)
-};
 
 template <int XIN>
 __global__ void __launch_bounds__(RELAX_NTHREADS) k_xfwd(XfArgs a)
@@ -1378,16 +1316,6 @@ __global__ void __launch_bounds__(RW *N2, (RW * N2 <= 128) ? 8 : 4) k_xfwd_reg(c
 }
 
 
-// pass 2 / 4: complex transform along x2 for a tile of x1 wavenumbers
-struct YArgs {
-    Grid g;
-    float2 *S;
-    FftPlan py;
-    int tw;            // tile width (k1 columns)
-    int nbody;         // body planes [0, nbody)
-    int traction;      // also the traction plane (index nbody of blockIdx.y)
-    const struct YArgs *tab;   // batched launch: one entry per member (blockIdx.y)
-};
 
 template <int SIGN>
 __global__ void __launch_bounds__(RELAX_NTHREADS) k_ypass(YArgs a)
@@ -1402,13 +1330,13 @@ __global__ void __launch_bounds__(RELAX_NTHREADS) k_ypass(YArgs a)
     const size_t base = sidx(g, c, p, 0, k1t);
     for (int t = threadIdx.x; t < n * TW; t += blockDim.x) {
         const int i2 = t / TW, col = t % TW;
-        A[t] = col < ncol ? a.S[base + (size_t)i2 * g.K1 + col] : make_float2(0.f, 0.f);
+        A[t] = col < ncol ? a.S[base + (size_t)i2 * g.KP + col] : make_float2(0.f, 0.f);
     }
     __syncthreads();
     float2 *R = fft_smem<SIGN>(A, B, a.py, TW, TW, 1);
     for (int t = threadIdx.x; t < n * TW; t += blockDim.x) {
         const int i2 = t / TW, col = t % TW;
-        if (col < ncol) a.S[base + (size_t)i2 * g.K1 + col] = R[t];
+        if (col < ncol) a.S[base + (size_t)i2 * g.KP + col] = R[t];
     }
 }
 
@@ -1422,15 +1350,6 @@ __global__ void __launch_bounds__(RELAX_NTHREADS) k_ypass(YArgs a)
 //   cerrutimodified (src/green.f90:520-612; per-column coefficients FP64),
 //   inverse transform along x3, planes [0, nout) written back.
 // ------------------------------------------------------------------------
-struct ZArgs {
-    Grid g;
-    float2 *S;
-    FftPlan pz;
-    int tw, nin, nout;
-    float ratio1, ratio2;            // elastic response constants
-    double lambda, mu, gam;
-    const struct ZArgs *tab;         // batched launch: one entry per member (blockIdx.y)
-};
 
 __global__ void __launch_bounds__(RELAX_NTHREADS) k_zspec(ZArgs a)
 {
@@ -1603,18 +1522,18 @@ __global__ void __launch_bounds__(CW *N2, (N1 == 16 && N2 == 8) ? 1 : (N1 == 16 
     extern __shared__ float2 smy[];
     const Grid &g = a.g;
     const int c = threadIdx.x % CW, t = threadIdx.x / CW;
-    // columns (component, plane, k1) flattened: f = (cp np + pi) K1 + k1
+    // columns (component, plane, k1) flattened: f = (cp np + pi) KP + k1
     const int np = a.nbody + a.traction;
     const int f = blockIdx.x * CW + c;
-    const bool ok = f < 3 * np * g.K1;
-    const int cp = ok ? f / (np * g.K1) : 0, rem = ok ? f % (np * g.K1) : 0;
-    const int pi = rem / g.K1, k1c = rem % g.K1;
+    const bool ok = f < 3 * np * g.KP;
+    const int cp = ok ? f / (np * g.KP) : 0, rem = ok ? f % (np * g.KP) : 0;
+    const int pi = rem / g.KP, k1c = rem % g.KP;
     const int p = (a.traction && pi == a.nbody) ? g.sx3 : pi;
     const size_t base = sidx(g, cp, p, 0, k1c);
     float2 x[N1];
 #pragma unroll
     for (int j1 = 0; j1 < N1; j1++)
-        x[j1] = ok ? a.S[base + (size_t)(N2 * j1 + t) * g.K1] : make_float2(0.f, 0.f);
+        x[j1] = ok ? a.S[base + (size_t)(N2 * j1 + t) * g.KP] : make_float2(0.f, 0.f);
     RDft<N1, SIGN>::run(x);
 #pragma unroll
     for (int k1 = 1; k1 < N1; k1++)
@@ -1631,305 +1550,11 @@ __global__ void __launch_bounds__(CW *N2, (N1 == 16 && N2 == 8) ? 1 : (N1 == 16 
         RDft<N2, SIGN>::run(y);
         if (ok) {
 #pragma unroll
-            for (int k2 = 0; k2 < N2; k2++) a.S[base + (size_t)(k1 + N1 * k2) * g.K1] = y[k2];
+            for (int k2 = 0; k2 < N2; k2++) a.S[base + (size_t)(k1 + N1 * k2) * g.KP] = y[k2];
         }
     }
     (void)n;
 }
-
-// pass 3, register/shared-memory version.  The three components of CW
-// columns stay in shared memory (U[cp][k1][j2][c]) between the phases, so a
-// thread holds one N1 or 3 x N2 group at a time.  PRUNED: input planes
-// [n/2, n) are zero and only output planes [0, n/2) are wanted (the step's
-// Green's functions); otherwise nin/nout are honoured.
-constexpr int ZCOL = 26;   // floats of per-column constants in k_zspec_sm
-
-template <int N1, int N2, int CW, bool PRUNED, bool BATCH = false>
-__global__ void __launch_bounds__(CW *N2, (CW * N2 >= 256) ? 2 : 4) k_zspec_sm(const __grid_constant__ ZArgs a0)
-{
-    pdl_enter();
-    const ZArgs &a = BATCH ? a0.tab[blockIdx.y] : a0;
-    constexpr int n = N1 * N2, Q = N1 / N2;
-    static_assert(N1 % N2 == 0, "N1 must be a multiple of N2");
-    extern __shared__ float2 smz[];
-    float2 *U = smz;                                                   // [3][N1][N2][CW]
-    float *red = reinterpret_cast<float *>(smz + 3 * n * CW);          // [N2][12][CW]
-    // per column, ZCOL floats: the Cerruti coefficients cc[14], the surface
-    // traction (6 floats), then beta, c0, 1/den as doubles (float offset 20)
-    float *colc = red + N2 * 12 * CW;                                  // [CW][ZCOL]
-    const Grid &g = a.g;
-    const int c = threadIdx.x % CW, t = threadIdx.x / CW;
-    // columns (k1, k2) flattened over the plane: col = k2 K1 + k1
-    const int col = blockIdx.x * CW + c;
-    const bool ok = col < g.sx2 * g.K1;
-    const int k2i = ok ? col / g.K1 : 0, k1c = ok ? col % g.K1 : 0;
-    const double PI2 = 6.28318530717958623199592693708837032318;
-    const double inv_l3 = 1.0 / (n * g.dx3);
-    auto uidx = [&](int cp, int k1, int j) { return ((cp * N1 + k1) * N2 + j) * CW + c; };
-
-    // forward stage A: all loads first, then the three transforms
-    constexpr int NL = PRUNED ? N1 / 2 : N1;
-    float2 x[3][NL];
-#pragma unroll
-    for (int cp = 0; cp < 3; cp++)
-#pragma unroll
-        for (int j1 = 0; j1 < NL; j1++) {
-            const int i3 = N2 * j1 + t;
-            const bool ld = ok && (PRUNED || i3 < a.nin);
-            x[cp][j1] = ld ? a.S[sidx(g, cp, i3, k2i, k1c)] : make_float2(0.f, 0.f);
-        }
-    // while those loads are in flight, one thread per column reads the
-    // surface traction and forms the column's data-independent FP64
-    // constants of cerrutisolmodified (src/green.f90:578-609): beta =
-    // 2 pi |k|, c0 = 1/(2 mu beta^3), 1/den = 1/(2 alpha mu beta^4 (1 + gam/beta))
-    if (t == N2 - 1) {
-        float *cc = colc + c * ZCOL;
-        if (ok) {
-#pragma unroll
-            for (int cp = 0; cp < 3; cp++) {
-                const float2 tc = a.S[sidx(g, cp, g.sx3, k2i, k1c)];
-                cc[14 + 2 * cp] = tc.x;
-                cc[15 + 2 * cp] = tc.y;
-            }
-        }
-        double *cd = reinterpret_cast<double *>(cc + 20);
-        const double k1d = (double)k1c / (g.sx1 * g.dx1);
-        const double k2d = (k2i < g.sx2 / 2) ? (double)k2i / (g.sx2 * g.dx2) : -(double)(g.sx2 - k2i) / (g.sx2 * g.dx2);
-        if (ok && !(k1d == 0.0 && k2d == 0.0)) {
-            const double alpha = (a.lambda + a.mu) / (a.lambda + 2.0 * a.mu);
-            const double beta = PI2 * sqrt(k1d * k1d + k2d * k2d);
-            const double h = a.gam / beta;
-            cd[0] = beta;
-            cd[1] = 1.0 / (2.0 * a.mu * beta * beta * beta);
-            cd[2] = 1.0 / (2.0 * alpha * a.mu * beta * beta * beta * beta * (1 + h));
-        }
-    }
-    {
-        float2 tw[N1];   // W_n^(t k1), shared by the three components
-#pragma unroll
-        for (int k1 = 0; k1 < N1; k1++) tw[k1] = twn<-1>(a.pz.tw, t * k1);
-#pragma unroll
-        for (int cp = 0; cp < 3; cp++) {
-            float2 z[N1];
-#pragma unroll
-            for (int j1 = 0; j1 < N1; j1++) z[j1] = j1 < NL ? x[cp][j1] : make_float2(0.f, 0.f);
-            RDft<N1, -1>::run(z);
-#pragma unroll
-            for (int k1 = 0; k1 < N1; k1++) U[uidx(cp, k1, t)] = k1 ? cmul(z[k1], tw[k1]) : z[k1];
-        }
-    }
-    __syncthreads();
-
-    // stage B, elastic response, surface-traction moments
-    const double k1v = (double)k1c / (g.sx1 * g.dx1);
-    const double k2v = (k2i < g.sx2 / 2) ? (double)k2i / (g.sx2 * g.dx2) : -(double)(g.sx2 - k2i) / (g.sx2 * g.dx2);
-    const float k1f = (float)k1v, k2f = (float)k2v;
-    const double alpha = (a.lambda + a.mu) / (a.lambda + 2.0 * a.mu);
-    // elasticresponse as u = A c - B k (k.c) with A = ratio1 (1 + ratio2) / r2,
-    // B = ratio1 / r2^2 (src/green.f90:78-90 rearranged); surface traction
-    // from the FP64 sums Sk_i = sum k3 u_i and S_i = sum u_i over k3
-    const float ra = a.ratio1 * (1.f + a.ratio2);
-    const float il3f = (float)inv_l3;   // k3 = jw / (n dx3)
-    // FP32 partial sums of jw u_i (k3 = jw / (n dx3)) and of u_i over this
-    // thread's k3; the reference accumulates these in REAL*4 over all k3
-    // (src/green.f90:365-367)
-    float acc[12] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-        const int k1 = t + N2 * q;
-        // SEQ (N2 >= 16): one component's DFT at a time, back to the
-        // thread's own slots of U, so that 3 N2 values never sit in
-        // registers together; otherwise the three stay in registers
-        constexpr bool SEQ = N2 >= 16;
-        float2 y[SEQ ? 1 : 3][N2];
-#pragma unroll
-        for (int cp = 0; cp < 3; cp++) {
-            float2 *v = y[SEQ ? 0 : cp];
-#pragma unroll
-            for (int jj = 0; jj < N2; jj++) v[jj] = U[uidx(cp, k1, jj)];
-            RDft<N2, -1>::run(v);
-            if (SEQ) {
-#pragma unroll
-                for (int jj = 0; jj < N2; jj++) U[uidx(cp, k1, jj)] = v[jj];
-            }
-        }
-#pragma unroll
-        for (int k2 = 0; k2 < N2; k2++) {
-            const int j = k1 + N1 * k2;
-            const int jw = j < n / 2 ? j : j - n;
-            const float w = (float)jw;
-            const float k3f = w * il3f;
-            const float2 c1 = SEQ ? U[uidx(0, k1, k2)] : y[0][k2];
-            const float2 c2 = SEQ ? U[uidx(1, k1, k2)] : y[SEQ ? 0 : 1][k2];
-            const float2 c3 = SEQ ? U[uidx(2, k1, k2)] : y[SEQ ? 0 : 2][k2];
-            const float r2 = k1f * k1f + k2f * k2f + k3f * k3f;
-            float2 u1, u2, u3;
-            if (r2 > 0.f) {
-                const float ir2 = rcp_fast(r2);
-                const float A = ra * ir2, B = a.ratio1 * ir2 * ir2;
-                const float kcr = k1f * c1.x + k2f * c2.x + k3f * c3.x;
-                const float kci = k1f * c1.y + k2f * c2.y + k3f * c3.y;
-                u1 = make_float2(A * c1.x - B * k1f * kcr, A * c1.y - B * k1f * kci);
-                u2 = make_float2(A * c2.x - B * k2f * kcr, A * c2.y - B * k2f * kci);
-                u3 = make_float2(A * c3.x - B * k3f * kcr, A * c3.y - B * k3f * kci);
-            } else {
-                u1 = u2 = u3 = make_float2(0.f, 0.f);
-            }
-            U[uidx(0, k1, k2)] = u1;
-            U[uidx(1, k1, k2)] = u2;
-            U[uidx(2, k1, k2)] = u3;
-            acc[0] += w * u1.x; acc[1] += w * u1.y; acc[2] += w * u2.x;
-            acc[3] += w * u2.y; acc[4] += w * u3.x; acc[5] += w * u3.y;
-            acc[6] += u1.x; acc[7] += u1.y; acc[8] += u2.x; acc[9] += u2.y; acc[10] += u3.x; acc[11] += u3.y;
-        }
-    }
-#pragma unroll
-    for (int qq = 0; qq < 12; qq++) red[(t * 12 + qq) * CW + c] = acc[qq];
-    __syncthreads();
-    if (t == 0) {
-        double s[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-        for (int tt = 0; tt < N2; tt++)
-            for (int qq = 0; qq < 12; qq++) s[qq] += (double)red[(tt * 12 + qq) * CW + c];
-        for (int qq = 0; qq < 6; qq++) s[qq] *= inv_l3;
-        float *cc = colc + c * ZCOL;
-        const double *cd = reinterpret_cast<const double *>(cc + 20);
-        float tr[6];
-#pragma unroll
-        for (int qq = 0; qq < 6; qq++) tr[qq] = cc[14 + qq];
-#pragma unroll
-        for (int qq = 0; qq < 14; qq++) cc[qq] = 0.f;
-        if (ok && !(k1v == 0.0 && k2v == 0.0)) {
-            // surfacetractioncowling (src/green.f90:356-366): i 2pi (...) - grav u3
-            const double modulus = a.lambda + 2.0 * a.mu;
-            const double grav = 2.0 * a.mu * alpha * a.gam;
-            const double a1r = a.mu * (s[0] + k1v * s[10]), a1i = a.mu * (s[1] + k1v * s[11]);
-            const double a2r = a.mu * (s[2] + k2v * s[10]), a2i = a.mu * (s[3] + k2v * s[11]);
-            const double a3r = modulus * s[4] + a.lambda * (k1v * s[6] + k2v * s[8]);
-            const double a3i = modulus * s[5] + a.lambda * (k1v * s[7] + k2v * s[9]);
-            const double sum[6] = {-PI2 * a1i, PI2 * a1r, -PI2 * a2i, PI2 * a2r,
-                                   -PI2 * a3i - grav * s[10], PI2 * a3r - grav * s[11]};
-            const double id = inv_l3;   // 1 / (n dx3)
-            double p[6];
-#pragma unroll
-            for (int qq = 0; qq < 6; qq++) p[qq] = (double)tr[qq] - sum[qq] * id;
-            // cerrutisolmodified (src/green.f90:578-609) written as
-            // u_i += fi (P_i + g R_i), g = 2 pi k3 fi, with per-column P_i, R_i
-            const double beta = cd[0], c0 = cd[1], iden = cd[2];
-            const double b1r = p[0] * c0, b1i = p[1] * c0, b2r = p[2] * c0, b2i = p[3] * c0;
-            const double qr = PI2 * k1v * p[0] + PI2 * k2v * p[2], qi = PI2 * k1v * p[1] + PI2 * k2v * p[3];
-            const double b3r = (beta * p[4] + (1.0 - alpha) * qi) * iden;
-            const double b3i = (beta * p[5] - (1.0 - alpha) * qr) * iden;
-            const double Qr = b1r * k1v + b2r * k2v, Qi = b1i * k1v + b2i * k2v;
-            const double ialpha = (a.lambda + 2.0 * a.mu) / (a.lambda + a.mu);   // 1 / alpha
-            const double ab = alpha * beta * PI2, er = 1.0 - ialpha, ab2 = -alpha * beta * beta;
-            const double ap = alpha * PI2 * PI2, bb = 2.0 * beta * beta;
-            // P_1 = i k1 ab er b3 - 2 beta^2 b1' + ap k1 Q ; R_1 = k1 ab b3 - i ap k1 Q
-            cc[0] = (float)(-k1v * ab * er * b3i - bb * b1r + ap * k1v * Qr);
-            cc[1] = (float)(k1v * ab * er * b3r - bb * b1i + ap * k1v * Qi);
-            cc[2] = (float)(k1v * ab * b3r + ap * k1v * Qi);
-            cc[3] = (float)(k1v * ab * b3i - ap * k1v * Qr);
-            cc[4] = (float)(-k2v * ab * er * b3i - bb * b2r + ap * k2v * Qr);
-            cc[5] = (float)(k2v * ab * er * b3r - bb * b2i + ap * k2v * Qi);
-            cc[6] = (float)(k2v * ab * b3r + ap * k2v * Qi);
-            cc[7] = (float)(k2v * ab * b3i - ap * k2v * Qr);
-            // P_3 = ab2 b3 / alpha ; R_3 = -i ab2 b3 + alpha beta 2pi Q
-            cc[8] = (float)(ab2 * b3r * ialpha);
-            cc[9] = (float)(ab2 * b3i * ialpha);
-            cc[10] = (float)(ab2 * b3i + alpha * beta * PI2 * Qr);
-            cc[11] = (float)(-ab2 * b3r + alpha * beta * PI2 * Qi);
-            cc[12] = (float)beta;
-            cc[13] = 1.f;
-        }
-    }
-    __syncthreads();
-
-    // Cerruti correction, inverse stage B, twiddle (in place in U)
-    {
-        float cc[14];
-#pragma unroll
-        for (int qq = 0; qq < 14; qq++) cc[qq] = colc[c * ZCOL + qq];
-        const bool cerr = cc[13] != 0.f;
-        const float pi2 = 6.28318530717958623f;
-        const float beta = cc[12], b2 = beta * beta;
-        const float il3 = (float)inv_l3;
-#pragma unroll
-        for (int q = 0; q < Q; q++) {
-            const int k1 = t + N2 * q;
-            constexpr bool SEQ = N2 >= 16;   // as in stage B
-            float2 y[SEQ ? 1 : 3][N2];
-            if (!SEQ || cerr) {
-#pragma unroll
-                for (int k2 = 0; k2 < N2; k2++) {
-                    float2 u1 = U[uidx(0, k1, k2)], u2 = U[uidx(1, k1, k2)], u3 = U[uidx(2, k1, k2)];
-                    if (cerr) {
-                        const int j = k1 + N1 * k2;
-                        const float k3f = (float)(j < n / 2 ? j : j - n) * il3;
-                        const float fi = (2.f * beta) * rcp_fast((pi2 * pi2) * (k3f * k3f) + b2);
-                        const float gg = pi2 * k3f * fi;
-                        u1.x += fi * (cc[0] + gg * cc[2]); u1.y += fi * (cc[1] + gg * cc[3]);
-                        u2.x += fi * (cc[4] + gg * cc[6]); u2.y += fi * (cc[5] + gg * cc[7]);
-                        u3.x += fi * (cc[8] + gg * cc[10]); u3.y += fi * (cc[9] + gg * cc[11]);
-                    }
-                    if (SEQ) {
-                        U[uidx(0, k1, k2)] = u1; U[uidx(1, k1, k2)] = u2; U[uidx(2, k1, k2)] = u3;
-                    } else {
-                        y[0][k2] = u1; y[SEQ ? 0 : 1][k2] = u2; y[SEQ ? 0 : 2][k2] = u3;
-                    }
-                }
-            }
-            float2 tw[N2];   // W_n^(-jj k1), shared by the three components
-#pragma unroll
-            for (int jj = 0; jj < N2; jj++) tw[jj] = twn<+1>(a.pz.tw, jj * k1);
-#pragma unroll
-            for (int cp = 0; cp < 3; cp++) {
-                float2 *v = y[SEQ ? 0 : cp];
-                if (SEQ) {
-#pragma unroll
-                    for (int jj = 0; jj < N2; jj++) v[jj] = U[uidx(cp, k1, jj)];
-                }
-                RDft<N2, +1>::run(v);
-#pragma unroll
-                for (int jj = 0; jj < N2; jj++) U[uidx(cp, k1, jj)] = jj ? cmul(v[jj], tw[jj]) : v[jj];
-            }
-        }
-    }
-    __syncthreads();
-
-    // inverse stage A and store
-#pragma unroll
-    for (int cp = 0; cp < 3; cp++) {
-        float2 z[N1];
-#pragma unroll
-        for (int k1 = 0; k1 < N1; k1++) z[k1] = U[uidx(cp, k1, t)];
-        RDft<N1, +1>::run(z);
-        if (ok) {
-#pragma unroll
-            for (int j1 = 0; j1 < N1; j1++) {
-                const int i3 = N2 * j1 + t;
-                if (PRUNED ? j1 < N1 / 2 : i3 < a.nout) a.S[sidx(g, cp, i3, k2i, k1c)] = z[j1];
-            }
-        }
-    }
-    (void)x;
-}
-
-// pass 5: C2R along x1, scaled by 2/(sx1 dx1 sx2 dx2 sx3 dx3), with the
-// field update out = base + coef * w  (fieldadd, src/elastic3d.f90:3774-3812)
-struct XiArgs {
-    Grid g;
-    const float2 *S;
-    FftPlan pm;
-    const float2 *tw1;
-    int rows;
-    float *out[3];
-    const float *base[3];
-    size_t rp, pp;           // pitches of out/base
-    const StepState *st;     // coef = cmul * Dt (or cmul when st is null)
-    float cmul, scale;
-    const struct XiArgs *tab;   // batched launch: one entry per member (blockIdx.z / 3)
-    float *vout[3];          // optional copy of the transformed field (the
-    int vplanes;             // velocity v) for planes i3 < vplanes, pitches rp/pp
-};
 
 __global__ void __launch_bounds__(RELAX_NTHREADS) k_xinv(XiArgs a)
 {
@@ -1982,16 +1607,16 @@ __global__ void __launch_bounds__(RW *N2, (N1 * N2 == 128) ? 3 : (N1 * N2 == 64)
     pdl_enter();
     const XiArgs &a = BATCH ? a0.tab[blockIdx.z / 3] : a0;
     // RW rows of one plane and component per block, N2 threads per row.
-    // (A) the block's spectrum rows, one contiguous run of RW*K1 values
+    // (A) the block's spectrum rows, one contiguous run of RW*KP values
     //     in S, are staged in shared memory with 16-byte loads;
     // (B) each row thread unpacks its stride-N2 inputs, transforms in
     //     registers and leaves the real row in shared memory;
     // (C) out = base + coef * scale * row with V-wide accesses (V = 4 for
     //     16-byte aligned rows, else 2).
-    constexpr int M = N1 * N2, Q = N1 / N2, N2P = N2 + 1, K1 = M + 1, NT = RW * N2, SX1 = 2 * M;
-    constexpr int RS0 = (N1 * N2P > K1 ? N1 * N2P : K1), RS = RS0 + ((8 - RS0 % 16) + 16) % 16;
+    constexpr int M = N1 * N2, Q = N1 / N2, N2P = N2 + 1, KP = M + 2, NT = RW * N2, SX1 = 2 * M;
+    constexpr int RS0 = (N1 * N2P > KP ? N1 * N2P : KP), RS = RS0 + ((8 - RS0 % 16) + 16) % 16;
     static_assert(N1 % N2 == 0, "N1 must be a multiple of N2");
-    static_assert(RS % 2 == 0 && (RW * K1) % 2 == 0, "float4 staging");
+    static_assert(RS % 2 == 0 && M % 2 == 0, "float4 staging");
     static_assert(V == 2 || V == 4, "V");
     extern __shared__ float2 smx[];
     const Grid &g = a.g;
@@ -2001,15 +1626,15 @@ __global__ void __launch_bounds__(RW *N2, (N1 * N2 == 128) ? 3 : (N1 * N2 == 64)
     // (A) rows i2b .. i2b+RW-1 are contiguous: sidx is linear in i2
     {
         const float4 *src = reinterpret_cast<const float4 *>(a.S + sidx(g, c, i3, i2b, 0));
-        constexpr int NF = RW * K1 / 2, ITS = (NF + NT - 1) / NT;
+        constexpr int NF = RW * KP / 2, ITS = (NF + NT - 1) / NT;
 #pragma unroll
         for (int it = 0; it < ITS; it++) {
             const int f = threadIdx.x + NT * it;
             if (f < NF) {
                 const float4 v = __ldg(src + f);
                 const int e0 = 2 * f, e1 = 2 * f + 1;
-                smx[(e0 / K1) * RS + e0 % K1] = make_float2(v.x, v.y);
-                smx[(e1 / K1) * RS + e1 % K1] = make_float2(v.z, v.w);
+                smx[(e0 / KP) * RS + e0 % KP] = make_float2(v.x, v.y);
+                smx[(e1 / KP) * RS + e1 % KP] = make_float2(v.z, v.w);
             }
         }
     }

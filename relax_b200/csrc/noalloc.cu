@@ -113,6 +113,7 @@ extern "C" int relax_op_green_noalloc(float *c1, float *c2, float *c3, float *t1
         return relax_noalloc_fail(RELAX_ERR_UNSUPPORTED, "grid: need sx1 >= 8, a multiple of 4, and even sx3");
     Grid g{};
     g.sx1 = sx1; g.sx2 = sx2; g.sx3 = sx3; g.sx3h = sx3 / 2; g.M = sx1 / 2; g.K1 = sx1 / 2 + 1;
+    g.KP = g.K1;   // the general kernels take any pitch
     g.dx1 = dx1; g.dx2 = dx2; g.dx3 = dx3; g.plane = (size_t)sx1 * sx2; g.nh = g.plane * g.sx3h;
     FftPlan pm{}, py{}, pz{};
     if (!factor(g.M, pm.r, &pm.nr) || !factor(sx2, py.r, &py.nr) || !factor(sx3, pz.r, &pz.nr))

@@ -27,6 +27,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "launch.cuh"
 #include "okada.cuh"
 #include "zspec_tc.cuh"
 
@@ -287,36 +288,6 @@ struct Prof {
 // register-resident column passes for the lengths they are instantiated for
 constexpr int kCW = 16;
 
-// Launch helpers of the register-resident passes.  `nm` members: with
-// nm > 1 the argument struct carries a device table (`tab`) with one entry
-// per member and the batched instantiation runs all members in one launch
-// (the member index is a spare grid dimension).
-template <typename K>
-static void set_smem(K kern, size_t sm)
-{
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-}
-
-// A launch with programmatic dependent launch allowed: the kernel (one that
-// enters through pdl_enter) may be scheduled while the previous kernel in the
-// stream finishes its last wave, and waits for it before touching memory.
-// Errors are left for cudaGetLastError, as with <<< >>>.
-template <typename... P, typename... A>
-static void launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t sm, cudaStream_t st, const A &...args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = sm;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    (void)cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
 template <int N1, int N2, int SIGN>
 static void launch_ypass_sign(const YArgs &ya, dim3 grid, size_t sm, int nm, cudaStream_t st)
 {
@@ -341,7 +312,7 @@ static cudaError_t launch_ypass_reg(const YArgs &ya, int sign, dim3 grid, int nm
 static bool ypass_reg(const YArgs &ya, int sign, cudaStream_t st, cudaError_t *e, int nm = 1)
 {
     // CW columns per block over the flattened (component, plane, k1) columns
-    const size_t ncol = (size_t)3 * (ya.nbody + ya.traction) * ya.g.K1;
+    const size_t ncol = (size_t)3 * (ya.nbody + ya.traction) * ya.g.KP;
     const dim3 grid((unsigned)((ncol + kCW - 1) / kCW));
     switch (ya.g.sx2) {
     case 32: *e = launch_ypass_reg<8, 4>(ya, sign, grid, nm, st); return true;
@@ -351,40 +322,6 @@ static bool ypass_reg(const YArgs &ya, int sign, cudaStream_t st, cudaError_t *e
     case 128: *e = launch_ypass_reg<16, 8>(ya, sign, grid, nm, st); return true;
     case 256: *e = launch_ypass_reg<16, 16>(ya, sign, grid, nm, st); return true;
     case 512: *e = launch_ypass_reg<32, 16>(ya, sign, grid, nm, st); return true;
-    default: return false;
-    }
-}
-
-template <int N1, int N2, bool PRUNED>
-static void launch_zspec_pr(const ZArgs &za, dim3 grid, size_t sm, int nm, cudaStream_t st)
-{
-    if (nm > 1) {
-        set_smem(k_zspec_sm<N1, N2, kCW, PRUNED, true>, sm);
-        launch_pdl(k_zspec_sm<N1, N2, kCW, PRUNED, true>, dim3(grid.x, nm), kCW * N2, sm, st, za);
-    } else {
-        set_smem(k_zspec_sm<N1, N2, kCW, PRUNED>, sm);
-        launch_pdl(k_zspec_sm<N1, N2, kCW, PRUNED>, grid, kCW * N2, sm, st, za);
-    }
-}
-
-template <int N1, int N2>
-static cudaError_t launch_zspec_reg(const ZArgs &za, dim3 grid, int nm, cudaStream_t st)
-{
-    const size_t sm = 3 * (size_t)N1 * N2 * kCW * sizeof(float2) + (size_t)N2 * 12 * kCW * sizeof(float) +
-                      (size_t)kCW * ZCOL * sizeof(float);
-    const bool pruned = 2 * za.nin == za.g.sx3 && 2 * za.nout == za.g.sx3;
-    if (pruned) launch_zspec_pr<N1, N2, true>(za, grid, sm, nm, st);
-    else launch_zspec_pr<N1, N2, false>(za, grid, sm, nm, st);
-    return cudaGetLastError();
-}
-
-static bool zspec_reg(const ZArgs &za, dim3 grid, cudaStream_t st, cudaError_t *e, int nm = 1)
-{
-    switch (za.g.sx3) {
-    case 96: *e = launch_zspec_reg<24, 4>(za, grid, nm, st); return true;
-    case 64: *e = launch_zspec_reg<8, 8>(za, grid, nm, st); return true;
-    case 128: *e = launch_zspec_reg<16, 8>(za, grid, nm, st); return true;
-    case 256: *e = launch_zspec_reg<16, 16>(za, grid, nm, st); return true;
     default: return false;
     }
 }
@@ -405,8 +342,8 @@ static void launch_xinv_v(const XiArgs &xi, int nout, size_t sm, int nm, cudaStr
 template <int N1, int N2>
 static cudaError_t launch_xinv_reg(const XiArgs &xi, int nout, int nm, cudaStream_t st)
 {
-    constexpr int RW = 32, N2P = N2 + 1, K1 = N1 * N2 + 1;
-    constexpr int RS0 = (N1 * N2P > K1 ? N1 * N2P : K1), RS = RS0 + ((8 - RS0 % 16) + 16) % 16;
+    constexpr int RW = 32, N2P = N2 + 1, KP = N1 * N2 + 2;
+    constexpr int RS0 = (N1 * N2P > KP ? N1 * N2P : KP), RS = RS0 + ((8 - RS0 % 16) + 16) % 16;
     const size_t sm = (size_t)RW * RS * sizeof(float2);
     // 16-byte output rows: float4 epilogue (the members of a batch share the layout)
     bool v4 = xi.rp % 4 == 0 && xi.pp % 4 == 0;
@@ -483,7 +420,7 @@ static bool reg_shape(const Grid &g)
     return (g.M == 32 || g.M == 64 || g.M == 96 || g.M == 128 || g.M == 256) && g.sx2 % 32 == 0 &&
            (g.sx2 == 32 || g.sx2 == 64 || g.sx2 == 96 || g.sx2 == 128 || g.sx2 == 192 || g.sx2 == 256 ||
             g.sx2 == 512) &&
-           (g.sx3 == 64 || g.sx3 == 96 || g.sx3 == 128 || g.sx3 == 256);
+           zspec_batch_length(g.sx3);
 }
 
 // the x3 pass with its DFT-64 sub-transforms on the tensor cores: 128-deep
@@ -494,7 +431,7 @@ static cudaError_t launch_zspec_tc(const ZArgs &za, int nsm, int *err, const uin
 {
     ZtcArgs t{};
     t.z = za;
-    t.ncol = za.g.sx2 * za.g.K1;
+    t.ncol = za.g.sx2 * za.g.KP;
     t.ntiles = (t.ncol + ZT_COLS - 1) / ZT_COLS;
     t.err = err;
     t.tab = tab;
@@ -526,13 +463,27 @@ struct Spectral {
     bool yreg = false;
     Grid g{};
     float2 *S = nullptr;
+    // in the buffer of S:
     float2 *tw = nullptr;          // tables for M, sx1, sx2, sx3
+    float4 *ptw = nullptr;         // those of sx3 as (cos, cos, sin, sin)
+    float4 *fg = nullptr;          // zspec_table for the planes that are written
     FftPlan pm{}, py{}, pz{};
     const float2 *tw1 = nullptr;
     int rows = 1, twy = 16, twz = 16;
     size_t smx = 0, smy = 0, smz = 0;
 
-    int init(const Grid &gg, cudaStream_t st)
+    // the limit of a general kernel, which contexts of all sizes share: one
+    // context's set-up must not lower it below another's need
+    template <typename K>
+    static cudaError_t smem_limit(K kern, size_t sm)
+    {
+        return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)std::max<size_t>(sm, 200 * 1024));
+    }
+
+    // planes: the planes that the Green's function writes at most (0: the
+    // transforms alone)
+    int init(const Grid &gg, cudaStream_t st, int planes)
     {
         g = gg;
         {
@@ -549,24 +500,37 @@ struct Spectral {
         const int ns[4] = {g.M, g.sx1, g.sx2, g.sx3};
         size_t tot = 0;
         for (int i = 0; i < 4; i++) tot += ns[i];
-        std::vector<float2> h(tot);
+        // one buffer: the spectrum, the correction table of the x3 pass, its
+        // twiddles as (cos, cos, sin, sin) and the plain tables
+        const size_t nrow = 3 * (size_t)(g.sx3 + 1) * g.sx2, nS = nrow * g.KP;
+        const size_t nfg = planes && zspec_length(g.sx3) ? 2 * zspec_table_stride(g) * planes : 0, np = 2 * (size_t)g.sx3;
+        std::vector<float2> h(np + tot);
         size_t off[4], o = 0;
         for (int i = 0; i < 4; i++) {
             off[i] = o;
             for (int j = 0; j < ns[i]; j++) {
                 const double a = -2.0 * M_PI * (double)j / (double)ns[i];
-                h[o + j] = make_float2((float)cos(a), (float)sin(a));
+                h[np + o + j] = make_float2((float)cos(a), (float)sin(a));
             }
             o += ns[i];
         }
-        TRY(dalloc(&tw, tot));
-        CK(cudaMemcpyAsync(tw, h.data(), tot * sizeof(float2), cudaMemcpyHostToDevice, st));
-        CK(cudaStreamSynchronize(st));
+        for (int j = 0; j < g.sx3; j++) {
+            const float2 w = h[np + off[3] + j];
+            h[2 * j] = make_float2(w.x, w.x);
+            h[2 * j + 1] = make_float2(w.y, w.y);
+        }
+        TRY(dalloc(&S, nS + nfg + h.size()));
+        fg = nfg ? reinterpret_cast<float4 *>(S + nS) : nullptr;
+        ptw = reinterpret_cast<float4 *>(S + nS + nfg);
+        tw = S + nS + nfg + np;
+        // (pageable memory: the call returns once the tables are staged)
+        CK(cudaMemcpyAsync(ptw, h.data(), h.size() * sizeof(float2), cudaMemcpyHostToDevice, st));
         pm.tw = tw + off[0];
         tw1 = tw + off[1];
         py.tw = tw + off[2];
         pz.tw = tw + off[3];
-        TRY(dalloc(&S, 3 * (size_t)(g.sx3 + 1) * g.sx2 * g.K1));
+        CK(cudaMemset2DAsync(S + g.K1, g.KP * sizeof(float2), 0, (g.KP - g.K1) * sizeof(float2), nrow, st));
+        if (fg) CK(zspec_table(g, fg, planes, st));
         // tile choices
         rows = 1;
         while (rows * 2 <= std::max(1, 1024 / g.M) && g.sx2 % (rows * 2) == 0) rows *= 2;
@@ -579,22 +543,23 @@ struct Spectral {
         const int P = RELAX_NTHREADS / twz;
         smz = 2 * (size_t)g.sx3 * 3 * twz * sizeof(float2) + (size_t)P * twz * 6 * sizeof(double) +
               (size_t)twz * 12 * sizeof(float);
-        CK(cudaFuncSetAttribute(k_xfwd<XIN_DIV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx));
-        CK(cudaFuncSetAttribute(k_xfwd<XIN_REAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx));
-        CK(cudaFuncSetAttribute(k_xinv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx));
-        CK(cudaFuncSetAttribute(k_ypass<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smy));
-        CK(cudaFuncSetAttribute(k_ypass<+1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smy));
-        CK(cudaFuncSetAttribute(k_zspec, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz));
+        CK(smem_limit(k_xfwd<XIN_DIV>, smx));
+        CK(smem_limit(k_xfwd<XIN_REAL>, smx));
+        CK(smem_limit(k_xinv, smx));
+        CK(smem_limit(k_ypass<-1>, smy));
+        CK(smem_limit(k_ypass<+1>, smy));
+        CK(smem_limit(k_zspec, smz));
         return RELAX_OK;
     }
 
     void release(bool idle = false)
     {
         if (S) dfree(S, idle);
-        if (tw) dfree(tw, idle);
         if (ztab) dfree(ztab, idle);
         S = nullptr;
         tw = nullptr;
+        ptw = nullptr;
+        fg = nullptr;
         ztab = nullptr;
     }
 
@@ -611,7 +576,9 @@ struct Spectral {
     ZArgs zargs(int nin, int nout, double lambda, double mu, double gam, int tile) const
     {
         ZArgs za{};
-        za.g = g; za.S = S; za.pz = pz; za.tw = tile; za.nin = nin; za.nout = nout;
+        za.g = g; za.S = S; za.pz = pz; za.pt = ptw; za.tw = tile; za.nin = nin; za.nout = nout;
+        za.ik1 = 1.0 / (g.sx1 * g.dx1); za.ik2 = 1.0 / (g.sx2 * g.dx2); za.ik3 = 1.0 / (g.sx3 * g.dx3);
+        za.fg = fg; za.fgs = zspec_table_stride(g);
         za.ratio1 = (float)((lambda + mu) / (lambda + 2.0 * mu) / mu / (4.0 * M_PI * M_PI));
         za.ratio2 = (float)(mu / (lambda + mu));
         za.lambda = lambda; za.mu = mu; za.gam = gam;
@@ -659,8 +626,8 @@ struct Spectral {
             if (re != cudaSuccess) return fail(RELAX_ERR_CUDA, "k_zspec_tc: %s", cudaGetErrorString(re));
             zr = true;
         }
-        if (use_reg && !zr) {
-            TIMED(prof, ST_ZSPEC, st, (zr = zspec_reg(za, dim3((g.sx2 * g.K1 + kCW - 1) / kCW), st, &re)));
+        if (use_reg && fg && !zr) {
+            TIMED(prof, ST_ZSPEC, st, (zr = zspec_reg(za, st, &re)));
             if (re != cudaSuccess) return fail(RELAX_ERR_CUDA, "k_zspec_reg: %s", cudaGetErrorString(re));
         }
         if (!zr) {
@@ -704,7 +671,7 @@ static int make_grid(Grid &g, int sx1, int sx2, int sx3, double dx1, double dx2,
         return fail(RELAX_ERR_UNSUPPORTED, "grid %dx%dx%d: FFT lengths must be products of 2 and 3", sx1, sx2, sx3);
     if (!(dx1 > 0 && dx2 > 0 && dx3 > 0)) return fail(RELAX_ERR_ARG, "non-positive sampling");
     g.sx1 = sx1; g.sx2 = sx2; g.sx3 = sx3; g.sx3h = sx3 / 2;
-    g.M = sx1 / 2; g.K1 = sx1 / 2 + 1;
+    g.M = sx1 / 2; g.K1 = sx1 / 2 + 1; g.KP = spectrum_pitch(g.K1);
     g.dx1 = dx1; g.dx2 = dx2; g.dx3 = dx3;
     g.plane = (size_t)sx1 * sx2;
     g.nh = g.plane * g.sx3h;
@@ -1069,7 +1036,7 @@ static int create(const relax_config *cfg, int device, relax_ctx *c)
     CK(cudaMemsetAsync(c->u, 0, 3 * nh * sizeof(float), c->st));
     CK(cudaMemsetAsync(c->vp, 0, 3 * nh * sizeof(float), c->st));
     CK(cudaMemsetAsync(c->gamma, 0, nh * sizeof(float), c->st));
-    TRY(c->sp.init(g, c->st));
+    TRY(c->sp.init(g, c->st, g.sx3h));
     c->sp.prof = &c->prof;
 
     // tau = -prestress (src/relax.f90:287-297)
@@ -3148,7 +3115,7 @@ extern "C" int relax_op_green(float *c1, float *c2, float *c3, float *t1, float 
     TRY(make_grid(g, sx1, sx2, sx3, dx1, dx2, dx3));
     cudaStream_t st = (cudaStream_t)stream;
     Spectral sp;
-    int rc = sp.init(g, st);
+    int rc = sp.init(g, st, sx3);
     if (rc != RELAX_OK) {
         sp.release();
         return rc;
@@ -3176,7 +3143,7 @@ extern "C" int relax_op_green_mixed(float *c1, float *c2, float *c3, float *t1, 
     cudaStream_t st = (cudaStream_t)stream;
     Spectral sp;
     int *err = nullptr;
-    int rc = sp.init(g, st);
+    int rc = sp.init(g, st, 0);
     if (rc == RELAX_OK) rc = dalloc(&err, 1);
     if (rc != RELAX_OK) {
         sp.release();
@@ -3297,11 +3264,11 @@ extern "C" int relax_op_fft3(float *data, int sx1, int sx2, int sx3, double dx1,
     if (!data) return fail(RELAX_ERR_ARG, "null data");
     if (sx1 < 4 || sx1 % 4 || !fft_size_ok(sx1 / 2) || !fft_size_ok(sx2) || !fft_size_ok(sx3))
         return fail(RELAX_ERR_UNSUPPORTED, "FFT sizes %dx%dx%d", sx1, sx2, sx3);
-    g.sx1 = sx1; g.sx2 = sx2; g.sx3 = sx3; g.sx3h = sx3 / 2; g.M = sx1 / 2; g.K1 = sx1 / 2 + 1;
+    g.sx1 = sx1; g.sx2 = sx2; g.sx3 = sx3; g.sx3h = sx3 / 2; g.M = sx1 / 2; g.K1 = sx1 / 2 + 1; g.KP = spectrum_pitch(g.K1);
     g.dx1 = dx1; g.dx2 = dx2; g.dx3 = dx3; g.plane = (size_t)sx1 * sx2; g.nh = g.plane * g.sx3h;
     cudaStream_t st = (cudaStream_t)stream;
     Spectral sp;
-    int rc = sp.init(g, st);
+    int rc = sp.init(g, st, 0);
     if (rc != RELAX_OK) {
         sp.release();
         return rc;
@@ -3681,7 +3648,7 @@ static int batch_green(relax_batch *b, const XiArgs &xi0)
         return fail(RELAX_ERR_CUDA, "batched x pass: %s", cudaGetErrorString(e));
     if (!ypass_reg(t.yf0, -1, b->st, &e, n) || e != cudaSuccess)
         return fail(RELAX_ERR_CUDA, "batched y pass: %s", cudaGetErrorString(e));
-    if (!zspec_reg(t.z0, dim3((g.sx2 * g.K1 + kCW - 1) / kCW), b->st, &e, n) || e != cudaSuccess)
+    if (!zspec_reg(t.z0, b->st, &e, n) || e != cudaSuccess)
         return fail(RELAX_ERR_CUDA, "batched z pass: %s", cudaGetErrorString(e));
     if (!ypass_reg(t.yi0, +1, b->st, &e, n) || e != cudaSuccess)
         return fail(RELAX_ERR_CUDA, "batched y pass: %s", cudaGetErrorString(e));

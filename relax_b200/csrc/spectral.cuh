@@ -1,0 +1,104 @@
+// spectral.cuh -- arguments and launchers of the five passes of the
+// Fourier-domain Green's function (x1 forward, x2, x3 with the elastic
+// response, x2 inverse, x1 inverse with the field update).
+#pragma once
+
+#include "common.cuh"
+
+namespace relax {
+
+// Derivatives along the periodic axes x1 and x2.  optimalfilter
+// (src/elastic3d.f90:846-907) takes the central difference
+// (w[i+1] - w[i-1]) / (2 dx) for sx <= 4 and sx >= 15, and the 7-point FIR
+// differentiator fir7 of src/kernel7.inc for 5 <= sx <= 14: sum over
+// l = 1..7 of (w[i+l] - w[i-l]) fir7(l) / dx, indexes periodic
+// (localstrain_ani, src/elastic3d.f90:1140-1178, and localdivergence_ani,
+// :1431-1470).  A Fir7 with n = 7 selects the filter, c[l-1] = fir7(l) / dx;
+// n = 0 the central difference.  Along x3, fir7 is selected for
+// 5 <= sx3/2 <= 14, but then every layer is a boundary layer of the filter
+// ((i3 > 7) and (i3 < sx3/2 - 6) is never true, stressupdate :975-976), so
+// the finite differences of localstrain_ani apply throughout.
+struct Fir7 {
+    int n;
+    float c[7];
+};
+
+enum { XIN_DIV = 0, XIN_REAL = 1 };
+
+// pass 1: R2C along x1
+struct XfArgs {
+    Grid g;
+    float2 *S;
+    FftPlan pm;              // complex length M = sx1/2
+    const float2 *tw1;       // exp(-2 pi i k / sx1)
+    int nin, rows;
+    int has_trac;            // blockIdx.y == nin is the traction plane
+    const float *m;          // XIN_DIV: 6 x nh moment
+    float k1, k2, k3, k3b;
+    Fir7 fx, fy;             // XIN_DIV: the x1, x2 differentiators (n = 7: fir7, k_xfwd only)
+    const float *in[3];      // XIN_REAL
+    size_t rp, pp;           // row / plane pitch (elements)
+    const float *tin[3];
+    size_t trp;
+    const float *tload;      // optional surface load added to t3 (sx1 x sx2)
+    float scale3, scale2;
+    const struct XfArgs *tab;   // batched launch: one entry per member (blockIdx.z)
+};
+
+// pass 2 / 4: complex transform along x2 for a tile of x1 wavenumbers
+struct YArgs {
+    Grid g;
+    float2 *S;
+    FftPlan py;
+    int tw;            // tile width (k1 columns)
+    int nbody;         // body planes [0, nbody)
+    int traction;      // also the traction plane (index nbody of blockIdx.y)
+    const struct YArgs *tab;   // batched launch: one entry per member (blockIdx.y)
+};
+
+// pass 3: the Green's function on x3 columns
+struct ZArgs {
+    Grid g;
+    float2 *S;
+    FftPlan pz;
+    const float4 *pt;                // pz.tw as (cos, cos, sin, sin)
+    int tw, nin, nout;
+    double ik1, ik2, ik3;            // wavenumber steps 1/(sx dx)
+    const float4 *fg;                // the correction's inverse transforms (zspec_table)
+    size_t fgs;                      // and their plane stride
+    float ratio1, ratio2;            // elastic response constants
+    double lambda, mu, gam;
+    const struct ZArgs *tab;         // batched launch: one entry per member (blockIdx.y)
+};
+
+// pass 5: C2R along x1 with the field update
+struct XiArgs {
+    Grid g;
+    const float2 *S;
+    FftPlan pm;
+    const float2 *tw1;
+    int rows;
+    float *out[3];
+    const float *base[3];
+    size_t rp, pp;           // pitches of out/base
+    const StepState *st;     // coef = cmul * Dt (or cmul when st is null)
+    float cmul, scale;
+    const struct XiArgs *tab;   // batched launch: one entry per member (blockIdx.z / 3)
+    float *vout[3];          // optional copy of the transformed field (the
+    int vplanes;             // velocity v) for planes i3 < vplanes, pitches rp/pp
+};
+
+// The register-resident passes: false when the grid's length has no
+// instantiation (the caller takes the general kernel).  nm > 1: one launch
+// for the nm members of a batch, whose arguments are args.tab.
+bool zspec_reg(const ZArgs &za, cudaStream_t st, cudaError_t *e, int nm = 1);
+// whether the x3 pass is instantiated for a length
+bool zspec_length(int sx3);
+// The table that zspec_reg reads for planes [0, planes): plane stride and
+// contents.  It depends on the grid alone.
+size_t zspec_table_stride(const Grid &g);
+cudaError_t zspec_table(const Grid &g, float4 *fg, int planes, cudaStream_t st);
+// lengths with batched instantiations of the x3 pass
+bool zspec_batch_length(int sx3);
+
+}  // namespace relax

@@ -1,0 +1,453 @@
+// zpass.cu -- the Fourier-domain Green's function on whole x3 columns.
+#include "launch.cuh"
+#include "pfft.cuh"
+#include "spectral.cuh"
+
+namespace relax {
+namespace {
+
+// Pass 3.  For CW pairs of neighbouring columns (x1 wavenumbers 2 kk and
+// 2 kk + 1 of one x2 wavenumber), all three components:
+//   forward transform along x3 (input planes [0, nin), zero below),
+//   elasticresponse (src/green.f90:51-101),
+//   surfacetractioncowling (src/green.f90:327-377) and p = t - p (:1082-1084),
+//   cerrutimodified (src/green.f90:520-612; per-column coefficients FP64),
+//   inverse transform along x3, planes [0, nout) written back.
+// PRUNED: input planes [n/2, n) are zero and only planes [0, n/2) are wanted
+// (the step's Green's functions); otherwise nin and nout are honoured.
+//
+// The pass reads and writes the spectrum once; what bounds it is instruction
+// issue and the latency of the transforms, so the columns go two by two
+// through f32x2 instructions (pfft.cuh).  The components stay in shared
+// memory between the phases (U[cp][k1][j][c]); 16 columns a block keep
+// 128-byte segments in global memory.  Shared memory limits an SM to 64
+// columns of 128 values, so a pair of columns takes N1 threads rather than
+// the N2 that one transform needs: in stage B a thread has one group of N2
+// values, in stage A the 3 N2 groups of N1 values are dealt out over the N1
+// threads.  The correction cerrutimodified adds fi (P_i + g R_i) to u_i with
+// per-column P, R and fi, g functions of k3 and the column alone, so its
+// inverse transforms come from a table of the plan (k_ztable) and it is
+// added after the inverse transform, to the planes that are written: the
+// values need not wait in shared memory for the sums that P and R take.
+// Measured against one column per thread with the correction applied to
+// every k3 (36 M warp instructions, now 21 M): 59.5 -> 46 us on the 256 x
+// 256 x 128 box, 502 -> 389 us on 512 x 512 x 256, 131 -> 103 us on 256^3;
+// against the general kernel 303 -> 60 us on 288 x 216 x 144.
+constexpr size_t zsmem(int n, int CW) { return 3 * (size_t)n * CW * 16 + (16 * 8 + 24 * 4) * 2 * CW; }
+// blocks on an SM: as many as shared memory holds, but no more than leave a
+// thread 128 registers (with fewer the transforms spill: 54 us instead of 46
+// for the 128-deep pass of the 256 x 256 x 128 box)
+constexpr int zblocks(int n, int N1, int CW)
+{
+    const int sm = (int)(233472 / (zsmem(n, CW) + 1024)), rg = 65536 / (128 * ((CW * N1 + 31) / 32 * 32));
+    return sm < rg ? sm : rg;
+}
+
+template <int N1, int N2, int CW, bool PRUNED, bool BATCH>
+__global__ void __launch_bounds__(CW *N1, zblocks(N1 *N2, N1, CW)) k_zpass(const __grid_constant__ ZArgs a0)
+{
+    pdl_enter();
+    const ZArgs &a = BATCH ? a0.tab[blockIdx.y] : a0;
+    constexpr int n = N1 * N2, NT = CW * N1, NC = 2 * CW;
+    constexpr int RA = (3 * N2 + N1 - 1) / N1;   // rounds of stage A
+    constexpr bool HOLD = N2 <= 6;               // stage B holds three components in registers, else two
+    static_assert((N2 >= 6 || HOLD) && NT >= NC, "shape");
+    static_assert(!PRUNED || N1 % 2 == 0, "the half-space ends between two groups");
+    extern __shared__ float2 U[];                             // real parts [3][N1][N2][CW], imaginary parts
+    constexpr int IM = 3 * n * CW;
+    double *sd = reinterpret_cast<double *>(U + 2 * IM);      // [12][NC] sums over k3
+    double *cd = sd + 12 * NC;                                // [4][NC] beta, c0, 1/den, fi g at k3 = -n/2
+    float *cc = reinterpret_cast<float *>(cd + 4 * NC);       // [3][6][NC] correction coefficients
+    float *tr = cc + 18 * NC;                                 // [6][NC] surface traction
+    const Grid &g = a.g;
+    const int c = threadIdx.x % CW, t = threadIdx.x / CW;
+    const int KP2 = g.KP / 2, npair = g.sx2 * KP2;
+    const int f = blockIdx.x * CW + c;
+    const bool ok = f < npair;
+    const size_t PS = (size_t)npair;                          // plane stride in pairs
+    float4 *S = reinterpret_cast<float4 *>(a.S) + (ok ? f : 0);
+    const size_t CS = (size_t)(g.sx3 + 1) * PS;               // component stride
+    // 8-byte accesses of a half-warp are two runs of CW pairs: the swizzle
+    // puts groups k1 and k1 + 1 into different halves of the banks (for odd
+    // N2 they are there already)
+    auto uidx = [&](int cp, int k1, int j) {
+        return ((cp * N1 + k1) * N2 + (N2 % 2 ? j : j ^ (k1 & 1))) * CW + c;
+    };
+    auto get = [&](int cp, int k1, int j) {
+        const int q = uidx(cp, k1, j);
+        return P2{U[q], U[q + IM]};
+    };
+    auto put = [&](int cp, int k1, int j, P2 v) {
+        const int q = uidx(cp, k1, j);
+        U[q] = v.r;
+        U[q + IM] = v.i;
+    };
+    const double PI2 = 6.28318530717958623199592693708837032318;
+
+    // forward stage A: the first round's loads, the next round's before the
+    // transform of the one that has arrived
+    constexpr int NL = PRUNED ? N1 / 2 : N1;
+    float4 x[NL];
+    auto load = [&](int r) {
+        const int task = r * N1 + t, cp = task / N2, j2 = task % N2;
+        if (3 * N2 % N1 && task >= 3 * N2) return;
+        const float4 *src = S + cp * CS + j2 * PS;
+#pragma unroll
+        for (int j1 = 0; j1 < NL; j1++)
+            x[j1] = PRUNED || N2 * j1 + j2 < a.nin ? src[N2 * j1 * PS] : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    load(0);
+    // while they are in flight, one thread per column (of the last warps,
+    // which have the fewest rounds) reads the surface traction and forms the
+    // column's data-independent FP64 constants of cerrutisolmodified
+    // (src/green.f90:578-609): beta = 2 pi |k|, c0 = 1/(2 mu beta^3), 1/den =
+    // 1/(2 alpha mu beta^4 (1 + gam/beta))
+    const int xc = threadIdx.x - (NT - NC);                   // column of the per-column work
+    const int xf = blockIdx.x * CW + xc / 2, xk2 = xf / KP2, xk1 = 2 * (xf - xk2 * KP2) + (xc & 1);
+    const bool xon = xc >= 0 && xf < npair && (xk1 | xk2) != 0;
+    if (xon) {
+#pragma unroll
+        for (int cp = 0; cp < 3; cp++) {
+            const float2 v = a.S[2 * (cp * CS + g.sx3 * PS + xf) + (xc & 1)];
+            tr[2 * cp * NC + xc] = v.x;
+            tr[(2 * cp + 1) * NC + xc] = v.y;
+        }
+        const double k1v = xk1 * a.ik1, k2v = (xk2 < g.sx2 / 2 ? xk2 : xk2 - g.sx2) * a.ik2;
+        const double alpha = (a.lambda + a.mu) / (a.lambda + 2.0 * a.mu);
+        const double beta = PI2 * sqrt(k1v * k1v + k2v * k2v);
+        const double h = a.gam / beta;
+        cd[xc] = beta;
+        cd[NC + xc] = 1.0 / (2.0 * a.mu * beta * beta * beta);
+        cd[2 * NC + xc] = 1.0 / (2.0 * alpha * a.mu * beta * beta * beta * beta * (1 + h));
+        const double k3n = -PI2 * (n / 2) * a.ik3, fin = 2.0 * beta / (k3n * k3n + beta * beta);
+        cd[3 * NC + xc] = k3n * fin * fin;
+    }
+#pragma unroll 1
+    for (int r = 0; r < RA; r++) {
+        const int task = r * N1 + t, cp = task / N2, j2 = task % N2;
+        if (3 * N2 % N1 && task >= 3 * N2) break;
+        P2 z[N1];
+#pragma unroll
+        for (int j1 = 0; j1 < NL; j1++) z[j1] = pair(x[j1]);
+        if (r + 1 < RA) load(r + 1);
+        PDft<N1, -1>::run(z, NL);
+#pragma unroll
+        for (int k1 = 0; k1 < N1; k1++) put(cp, k1, j2, z[k1]);
+    }
+    __syncthreads();
+
+    // stage B, elastic response, surface-traction moments.  elasticresponse
+    // as u = A c - B k (k.c) with A = ratio1 (1 + ratio2) / r2, B = ratio1 /
+    // r2^2 (src/green.f90:78-90 rearranged); per thread FP32 partial sums of
+    // jw u_i (k3 = jw / (n dx3)) and of u_i over its k3, combined in FP64
+    // (the reference accumulates them in REAL*4 over all k3,
+    // src/green.f90:365-367)
+    const int k2i = ok ? f / KP2 : 0, kk = ok ? f - k2i * KP2 : 0;
+    const float2 k1f = make_float2((float)(2 * kk * a.ik1), (float)((2 * kk + 1) * a.ik1));
+    const float k2s = (float)((k2i < g.sx2 / 2 ? k2i : k2i - g.sx2) * a.ik2);
+    const float2 k2f = f2(k2s);
+    const float2 k12 = fma2(k1f, k1f, f2(k2s * k2s));
+    const float il3 = (float)a.ik3;
+    const float2 ra = f2(a.ratio1 * (1.f + a.ratio2)), rb = f2(a.ratio1);
+    float2 acc[12];
+#pragma unroll
+    for (int q = 0; q < 12; q++) acc[q] = f2(0.f);
+    const float tf = (float)t;
+    auto response = [&](P2 &c1, P2 &c2, P2 &c3, int k2) {
+        // j = t + N1 k2 in the upper half is j - n: known from k2 alone for even N2
+        const bool up = N2 % 2 ? t + N1 * k2 >= n / 2 : 2 * k2 >= N2;
+        const float w = tf + (float)(up ? N1 * k2 - n : N1 * k2), k3s = w * il3;
+        const float2 k3f = f2(k3s), wf = f2(w);
+        const float2 r2 = add2(k12, f2(k3s * k3s));
+        // zero only at k1 = k2 = k3 = 0 (in lane x): no displacement there
+        const float2 ir2 = make_float2(k2 == 0 && r2.x == 0.f ? 0.f : rcp_fast(r2.x), rcp_fast(r2.y));
+        const float2 A = mul2(ra, ir2), B = mul2(mul2(rb, ir2), ir2);
+        const float2 kr = mul2(B, fma2(k3f, c3.r, fma2(k2f, c2.r, mul2(k1f, c1.r))));
+        const float2 ki = mul2(B, fma2(k3f, c3.i, fma2(k2f, c2.i, mul2(k1f, c1.i))));
+        const float2 n1 = neg2(k1f), n2 = neg2(k2f), n3 = neg2(k3f);
+        c1 = {fma2(n1, kr, mul2(A, c1.r)), fma2(n1, ki, mul2(A, c1.i))};
+        c2 = {fma2(n2, kr, mul2(A, c2.r)), fma2(n2, ki, mul2(A, c2.i))};
+        c3 = {fma2(n3, kr, mul2(A, c3.r)), fma2(n3, ki, mul2(A, c3.i))};
+        acc[0] = fma2(wf, c1.r, acc[0]); acc[1] = fma2(wf, c1.i, acc[1]);
+        acc[2] = fma2(wf, c2.r, acc[2]); acc[3] = fma2(wf, c2.i, acc[3]);
+        acc[4] = fma2(wf, c3.r, acc[4]); acc[5] = fma2(wf, c3.i, acc[5]);
+        acc[6] = add2(acc[6], c1.r); acc[7] = add2(acc[7], c1.i);
+        acc[8] = add2(acc[8], c2.r); acc[9] = add2(acc[9], c2.i);
+        acc[10] = add2(acc[10], c3.r); acc[11] = add2(acc[11], c3.i);
+    };
+    P2 y[HOLD ? 3 : 2][N2];
+    {
+        W2 w[N2];   // W_n^(jj t)
+#pragma unroll
+        for (int jj = 1; jj < N2; jj++) w[jj] = w2(__ldg(a.pt + jj * t));
+#pragma unroll
+        for (int cp = 2; cp >= 0; cp--) {
+            P2 *v = y[HOLD ? cp : cp % 2];
+#pragma unroll
+            for (int jj = 0; jj < N2; jj++) v[jj] = get(cp, t, jj);
+#pragma unroll
+            for (int jj = 1; jj < N2; jj++) v[jj] = pmul<false>(v[jj], w[jj]);
+            PDft<N2, -1>::run(v);
+            if (!HOLD && cp == 2) {
+#pragma unroll
+                for (int jj = 0; jj < N2; jj++) put(cp, t, jj, v[jj]);
+            }
+        }
+    }
+#pragma unroll
+    for (int k2 = 0; k2 < N2; k2++) {
+        P2 c3 = HOLD ? y[HOLD ? 2 : 0][k2] : get(2, t, k2);
+        response(y[0][k2], y[1][k2], c3, k2);
+        if (HOLD) y[HOLD ? 2 : 0][k2] = c3;
+        else put(2, t, k2, c3);
+    }
+    // the partial sums, in the thread's own slots that hold nothing now
+    // (component 0; all three where they are in registers)
+    auto slot = [&](int q, int k1, int cc) {
+        const int cp = HOLD ? q % 3 : 0, im = HOLD ? q / 3 % 2 : q / 6, j = HOLD ? q / 6 : q % 6;
+        return im * IM + ((cp * N1 + k1) * N2 + j) * CW + cc;
+    };
+#pragma unroll
+    for (int q = 0; q < 12; q++) U[slot(q, t, c)] = acc[q];
+    __syncthreads();
+    // the sums over k3 in a fixed order, FP64: one (sum, column) per thread
+    for (int s = threadIdx.x; s < 12 * NC; s += NT) {
+        const int q = s / NC, col = s % NC;
+        const float *v = reinterpret_cast<const float *>(U + slot(q, 0, col / 2)) + (col & 1);
+        double sum = 0.0;
+#pragma unroll
+        for (int tt = 0; tt < N1; tt++) sum += (double)v[2 * tt * N2 * CW];
+        sd[s] = sum;
+    }
+    __syncthreads();
+    if (xc >= 0) {
+#pragma unroll
+        for (int qq = 0; qq < 18; qq++) cc[qq * NC + xc] = 0.f;
+        if (xon) {
+            double s[12];
+#pragma unroll
+            for (int qq = 0; qq < 12; qq++) s[qq] = qq < 6 ? sd[qq * NC + xc] * a.ik3 : sd[qq * NC + xc];
+            const double k1v = xk1 * a.ik1, k2v = (xk2 < g.sx2 / 2 ? xk2 : xk2 - g.sx2) * a.ik2;
+            const double alpha = (a.lambda + a.mu) / (a.lambda + 2.0 * a.mu);
+            // surfacetractioncowling (src/green.f90:356-366): i 2pi (...) - grav u3
+            const double modulus = a.lambda + 2.0 * a.mu;
+            const double grav = 2.0 * a.mu * alpha * a.gam;
+            const double a1r = a.mu * (s[0] + k1v * s[10]), a1i = a.mu * (s[1] + k1v * s[11]);
+            const double a2r = a.mu * (s[2] + k2v * s[10]), a2i = a.mu * (s[3] + k2v * s[11]);
+            const double a3r = modulus * s[4] + a.lambda * (k1v * s[6] + k2v * s[8]);
+            const double a3i = modulus * s[5] + a.lambda * (k1v * s[7] + k2v * s[9]);
+            const double sum[6] = {-PI2 * a1i, PI2 * a1r, -PI2 * a2i, PI2 * a2r,
+                                   -PI2 * a3i - grav * s[10], PI2 * a3r - grav * s[11]};
+            double p[6];
+#pragma unroll
+            for (int qq = 0; qq < 6; qq++) p[qq] = (double)tr[qq * NC + xc] - sum[qq] * a.ik3;
+            // cerrutisolmodified (src/green.f90:578-609) written as
+            // u_i += fi (P_i + g R_i), g = 2 pi k3 fi, with per-column P_i, R_i
+            const double beta = cd[xc], c0 = cd[NC + xc], iden = cd[2 * NC + xc];
+            const double b1r = p[0] * c0, b1i = p[1] * c0, b2r = p[2] * c0, b2i = p[3] * c0;
+            const double qr = PI2 * k1v * p[0] + PI2 * k2v * p[2], qi = PI2 * k1v * p[1] + PI2 * k2v * p[3];
+            const double b3r = (beta * p[4] + (1.0 - alpha) * qi) * iden;
+            const double b3i = (beta * p[5] - (1.0 - alpha) * qr) * iden;
+            const double Qr = b1r * k1v + b2r * k2v, Qi = b1i * k1v + b2i * k2v;
+            const double ialpha = (a.lambda + 2.0 * a.mu) / (a.lambda + a.mu);   // 1 / alpha
+            const double ab = alpha * beta * PI2, er = 1.0 - ialpha, ab2 = -alpha * beta * beta;
+            const double ap = alpha * PI2 * PI2, bb = 2.0 * beta * beta;
+            const double gn = cd[3 * NC + xc];
+            auto coefs = [&](int cp, double pr, double pi, double rr, double ri) {
+                float *o = cc + 6 * cp * NC + xc;
+                o[0] = (float)pr; o[NC] = (float)pi; o[2 * NC] = (float)rr; o[3 * NC] = (float)ri;
+                o[4 * NC] = (float)(rr * gn); o[5 * NC] = (float)(ri * gn);
+            };
+            // P_1 = i k1 ab er b3 - 2 beta^2 b1' + ap k1 Q ; R_1 = k1 ab b3 - i ap k1 Q
+            coefs(0, -k1v * ab * er * b3i - bb * b1r + ap * k1v * Qr, k1v * ab * er * b3r - bb * b1i + ap * k1v * Qi,
+                k1v * ab * b3r + ap * k1v * Qi, k1v * ab * b3i - ap * k1v * Qr);
+            coefs(1, -k2v * ab * er * b3i - bb * b2r + ap * k2v * Qr, k2v * ab * er * b3r - bb * b2i + ap * k2v * Qi,
+                k2v * ab * b3r + ap * k2v * Qi, k2v * ab * b3i - ap * k2v * Qr);
+            // P_3 = ab2 b3 / alpha ; R_3 = -i ab2 b3 + alpha beta 2pi Q
+            coefs(2, ab2 * b3r * ialpha, ab2 * b3i * ialpha, ab2 * b3i + alpha * beta * PI2 * Qr,
+                -ab2 * b3r + alpha * beta * PI2 * Qi);
+        }
+    }
+
+    // inverse stage B and twiddle, back to the thread's own slots
+    {
+        W2 w[N2];
+#pragma unroll
+        for (int jj = 1; jj < N2; jj++) w[jj] = w2(__ldg(a.pt + jj * t));
+#pragma unroll
+        for (int cp = 0; cp < 3; cp++) {
+            P2 *v = y[HOLD ? cp : cp % 2];
+            if (!HOLD && cp == 2) {
+#pragma unroll
+                for (int k2 = 0; k2 < N2; k2++) v[k2] = get(2, t, k2);
+            }
+            PDft<N2, +1>::run(v);
+#pragma unroll
+            for (int jj = 0; jj < N2; jj++) put(cp, t, jj, jj ? pmul<true>(v[jj], w[jj]) : v[jj]);
+        }
+    }
+    __syncthreads();
+
+    // inverse stage A, the correction P F + R (i G + (-1)^i3 gn) (the last
+    // term, of the unpaired wavenumber -n/2, through one input of the
+    // transform over j1: (-1)^i3 is (-1)^j2, or (-1)^(j1 + j2) for odd N2),
+    // and store
+#pragma unroll 1
+    for (int r = 0; r < RA; r++) {
+        const int task = r * N1 + t, cp = task / N2, j2 = task % N2;
+        if (3 * N2 % N1 && task >= 3 * N2) break;
+        auto coef = [&](int q) { return *reinterpret_cast<const float2 *>(cc + (6 * cp + q) * NC + 2 * c); };
+        const float4 *fg = a.fg + (ok ? (k2i < g.sx2 / 2 ? k2i : g.sx2 - k2i) * KP2 + kk : 0) + j2 * a.fgs;
+        float4 FG[NL];
+#pragma unroll
+        for (int j1 = 0; j1 < NL; j1++)
+            FG[j1] = PRUNED || N2 * j1 + j2 < a.nout ? __ldg(fg + N2 * j1 * a.fgs) : make_float4(0.f, 0.f, 0.f, 0.f);
+        P2 z[N1];
+#pragma unroll
+        for (int k1 = 0; k1 < N1; k1++) z[k1] = get(cp, k1, j2);
+        const P2 e = {coef(4), coef(5)};
+        constexpr int KN = N2 % 2 ? N1 / 2 : 0;
+        z[KN] = j2 & 1 ? psub(z[KN], e) : padd(z[KN], e);
+        PDft<N1, +1>::run(z);
+        if (ok) {
+            const float2 pr = coef(0), pi = coef(1), rr = coef(2), mri = neg2(coef(3));
+            float4 *dst = S + cp * CS + j2 * PS;
+#pragma unroll
+            for (int j1 = 0; j1 < NL; j1++) {
+                const float2 F = make_float2(FG[j1].x, FG[j1].y), G = make_float2(FG[j1].z, FG[j1].w);
+                const P2 v = {fma2(mri, G, fma2(pr, F, z[j1].r)), fma2(rr, G, fma2(pi, F, z[j1].i))};
+                if (PRUNED || N2 * j1 + j2 < a.nout) dst[N2 * j1 * PS] = unpair(v);
+            }
+        }
+    }
+}
+
+// The table of the correction's inverse transforms: for every column of
+// x2 wavenumbers 0 .. sx2 - sx2/2 (the others by symmetry) and plane i3,
+//     F = sum_m fi cos(2 pi m i3 / n),  G = sum_m fi g sin(2 pi m i3 / n)
+// over the wavenumbers m of x3, fi = 2 beta / ((2 pi k3)^2 + beta^2), g = 2
+// pi k3 fi, summed in FP64; two columns in one entry (F, F, G, G).  A block
+// takes 16 columns of one row.
+constexpr int ZT_CW = 16;
+__global__ void __launch_bounds__(256) k_ztable(Grid g, float4 *fg, size_t fgs, int planes, double ik1, double ik2,
+                                                double ik3)
+{
+    extern __shared__ double zs[];
+    const int n = g.sx3, h = n / 2;
+    double *ct = zs, *f = zs + n, *fgn = f + ZT_CW * (h + 1);   // cos table, fi and fi g by (m, column)
+    const double PI2 = 6.28318530717958623199592693708837032318;
+    const int k1b = ZT_CW * blockIdx.x, k2 = blockIdx.y;
+    for (int j = threadIdx.x; j < n; j += blockDim.x) ct[j] = cospi(2.0 * j / n);
+    for (int s = threadIdx.x; s < ZT_CW * (h + 1); s += blockDim.x) {
+        const int m = s / ZT_CW, k1 = k1b + s % ZT_CW;
+        const double k1v = k1 * ik1, k2v = k2 * ik2, b2 = PI2 * PI2 * (k1v * k1v + k2v * k2v);
+        const double k3 = PI2 * m * ik3, fi = b2 > 0.0 ? 2.0 * sqrt(b2) / (k3 * k3 + b2) : 0.0;
+        f[s] = fi;
+        fgn[s] = k3 * fi * fi;
+    }
+    __syncthreads();
+    const int col = threadIdx.x % ZT_CW, k1 = k1b + col;
+    if (k1 >= g.KP) return;
+    for (int z = threadIdx.x / ZT_CW; z < planes; z += blockDim.x / ZT_CW) {
+        double F = f[col] + (z & 1 ? -1.0 : 1.0) * f[h * ZT_CW + col], G = 0.0;
+        int j = 0;   // m z mod n
+        for (int m = 1; m < h; m++) {
+            j += z;
+            if (j >= n) j -= n;
+            int q = j - n / 4;   // sin x = cos(x - pi/2) where n is a multiple of 4
+            if (q < 0) q += n;
+            const double sn = n % 4 ? sinpi(2.0 * j / n) : ct[q];
+            F += 2.0 * f[m * ZT_CW + col] * ct[j];
+            G += 2.0 * fgn[m * ZT_CW + col] * sn;
+        }
+        float *o = reinterpret_cast<float *>(fg + z * fgs + (size_t)k2 * (g.KP / 2) + k1 / 2);
+        o[k1 & 1] = (float)F;
+        o[2 + (k1 & 1)] = (float)G;
+    }
+}
+
+template <int N1, int N2, int CW, bool BATCH>
+void launch(const ZArgs &za, int nm, cudaStream_t st)
+{
+    const size_t sm = zsmem(N1 * N2, CW);
+    const int npair = za.g.sx2 * (za.g.KP / 2);
+    const dim3 grid((npair + CW - 1) / CW, nm);
+    const bool pruned = 2 * za.nin == za.g.sx3 && 2 * za.nout == za.g.sx3;
+    auto run = [&](void (*k)(ZArgs)) {
+        set_smem(k, sm);
+        launch_pdl(k, grid, CW * N1, sm, st, za);
+    };
+    if (pruned) run(k_zpass<N1, N2, CW, true, BATCH>);
+    else run(k_zpass<N1, N2, CW, false, BATCH>);
+}
+
+}  // namespace
+
+size_t zspec_table_stride(const Grid &g) { return (size_t)(g.sx2 - g.sx2 / 2 + 1) * (g.KP / 2); }
+
+cudaError_t zspec_table(const Grid &g, float4 *fg, int planes, cudaStream_t st)
+{
+    const size_t sm = (g.sx3 + 2 * ZT_CW * (size_t)(g.sx3 / 2 + 1)) * sizeof(double);
+    set_smem(k_ztable, sm);
+    const dim3 grid((g.KP + ZT_CW - 1) / ZT_CW, g.sx2 - g.sx2 / 2 + 1);
+    k_ztable<<<grid, 256, sm, st>>>(g, fg, zspec_table_stride(g), planes, 1.0 / (g.sx1 * g.dx1),
+                                    1.0 / (g.sx2 * g.dx2), 1.0 / (g.sx3 * g.dx3));
+    return cudaGetLastError();
+}
+
+bool zspec_batch_length(int sx3) { return sx3 == 64 || sx3 == 96 || sx3 == 128 || sx3 == 256; }
+
+// The lengths that are instantiated: the products of 2 and 3 up to 288, and
+// 384 and 512 (half the columns a block, for the same shared memory).  The
+// factors are those whose 3 N2 groups of stage A divide evenly over the N1
+// threads where there is a choice, N1 even.  Other lengths take k_zspec
+// (about 5 times slower: 303 against 60 us on a 288 x 216 x 144 box).
+bool zspec_length(int sx3)
+{
+    switch (sx3) {
+    case 24: case 32: case 36: case 48: case 54: case 64: case 72: case 96:
+    case 108: case 128: case 144: case 162: case 192: case 216: case 256: case 288: case 384: case 512:
+        return true;
+    default: return false;
+    }
+}
+
+bool zspec_reg(const ZArgs &za, cudaStream_t st, cudaError_t *e, int nm)
+{
+    if (nm > 1) {
+        switch (za.g.sx3) {
+        case 64: launch<8, 8, 8, true>(za, nm, st); break;
+        case 96: launch<12, 8, 8, true>(za, nm, st); break;
+        case 128: launch<16, 8, 8, true>(za, nm, st); break;
+        case 256: launch<16, 16, 8, true>(za, nm, st); break;
+        default: return false;
+        }
+        *e = cudaGetLastError();
+        return true;
+    }
+    switch (za.g.sx3) {
+    case 24: launch<6, 4, 8, false>(za, nm, st); break;
+    case 32: launch<8, 4, 8, false>(za, nm, st); break;
+    case 36: launch<6, 6, 8, false>(za, nm, st); break;
+    case 48: launch<12, 4, 8, false>(za, nm, st); break;
+    case 54: launch<18, 3, 8, false>(za, nm, st); break;
+    case 64: launch<8, 8, 8, false>(za, nm, st); break;
+    case 72: launch<12, 6, 8, false>(za, nm, st); break;
+    case 96: launch<12, 8, 8, false>(za, nm, st); break;
+    case 108: launch<18, 6, 8, false>(za, nm, st); break;
+    case 128: launch<16, 8, 8, false>(za, nm, st); break;
+    case 144: launch<12, 12, 8, false>(za, nm, st); break;
+    case 162: launch<18, 9, 8, false>(za, nm, st); break;
+    case 192: launch<24, 8, 8, false>(za, nm, st); break;
+    case 216: launch<24, 9, 8, false>(za, nm, st); break;
+    case 256: launch<16, 16, 8, false>(za, nm, st); break;
+    case 288: launch<24, 12, 8, false>(za, nm, st); break;
+    case 384: launch<24, 16, 4, false>(za, nm, st); break;
+    case 512: launch<32, 16, 4, false>(za, nm, st); break;
+    default: return false;
+    }
+    *e = cudaGetLastError();
+    return true;
+}
+
+}  // namespace relax

@@ -176,7 +176,7 @@ __device__ __forceinline__ void split2(float re, float im, uint32_t &hi, uint32_
 
 struct ZtcArgs {
     ZArgs z;          // grid, spectrum and elastic constants (z.nin = z.nout = 64)
-    int ncol;         // sx2 * K1 columns
+    int ncol;         // sx2 * KP columns
     int ntiles;       // ceil(ncol / 64)
     int *err;         // raised (1 << RELAX_ERR_CUDA) when a wait on the tensor cores times out
     const uint4 *tab; // k_ztc_tables: the DFT-64 matrix (hi, lo) in operand layout, then W128^n
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(ZT_THREADS, 1) k_zspec_tc(const __grid_constan
         return true;
     };
 
-    const size_t PS = (size_t)g.sx2 * g.K1;                 // plane stride of the spectrum
+    const size_t PS = (size_t)g.sx2 * g.KP;                 // plane stride of the spectrum
     const double inv_l3 = 1.0 / (128.0 * g.dx3);
     const float il3 = (float)inv_l3;
     const int lq = warp & 3, hv = warp >> 2;                // TMEM lane quarter, column half
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(ZT_THREADS, 1) k_zspec_tc(const __grid_constan
 #pragma unroll
             for (int q = 0; q < 12; q++) v[q] = 0.0;
             if (c < np) {
-                const int ck2 = pc / g.K1, ck1 = pc % g.K1;
+                const int ck2 = pc / g.KP, ck1 = pc % g.KP;
                 const double ck1v = (double)ck1 / (g.sx1 * g.dx1);
                 const double ck2v = (ck2 < g.sx2 / 2) ? (double)ck2 / (g.sx2 * g.dx2)
                                                       : -(double)(g.sx2 - ck2) / (g.sx2 * g.dx2);
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(ZT_THREADS, 1) k_zspec_tc(const __grid_constan
         // ---- elastic response, surface-traction partial sums ----------
         const int pcol = p0 + rcol;
         const bool colok = rcol < np;
-        const int k2i = colok ? pcol / g.K1 : 0, k1c = colok ? pcol % g.K1 : 0;
+        const int k2i = colok ? pcol / g.KP : 0, k1c = colok ? pcol % g.KP : 0;
         const double k1v = (double)k1c / (g.sx1 * g.dx1);
         const double k2v = (k2i < g.sx2 / 2) ? (double)k2i / (g.sx2 * g.dx2)
                                              : -(double)(g.sx2 - k2i) / (g.sx2 * g.dx2);
