@@ -1500,62 +1500,6 @@ __global__ void __launch_bounds__(RELAX_NTHREADS) k_zspec(ZArgs a)
 }
 
 
-// ------------------------------------------------------------------------
-// Register-resident variants of passes 2-4 (see rfft.cuh): columns of
-// length n = N1*N2, CW columns per block, N2 threads per column.
-// ------------------------------------------------------------------------
-
-// pass 2 / 4 along x2.  Register budgets as measured fastest: the 128-point
-// transform (128 threads a block) takes the registers it asks for (78
-// instead of 54-64 on 128 x 128 boxes), the 256-point one 3 blocks of 256
-// threads per SM (80 registers instead of 64: forward pass 30.4 -> 27.4 us
-// on the 256 x 256 x 128 box), the 512-point one 2 blocks per SM (128
-// registers instead of 85: 192 -> 187 us forward, 193 -> 185 us inverse on
-// the 512 x 512 x 256 box)
-template <int N1, int N2, int CW, int SIGN, bool BATCH = false>
-__global__ void __launch_bounds__(CW *N2, (N1 == 16 && N2 == 8) ? 1 : (N1 == 16 && N2 == 16) ? 3 : (N1 == 32) ? 2 : 0) k_ypass_reg(const __grid_constant__ YArgs a0)
-{
-    pdl_enter();
-    const YArgs &a = BATCH ? a0.tab[blockIdx.y] : a0;
-    constexpr int n = N1 * N2, Q = N1 / N2;
-    static_assert(N1 % N2 == 0, "N1 must be a multiple of N2");
-    extern __shared__ float2 smy[];
-    const Grid &g = a.g;
-    const int c = threadIdx.x % CW, t = threadIdx.x / CW;
-    // columns (component, plane, k1) flattened: f = (cp np + pi) KP + k1
-    const int np = a.nbody + a.traction;
-    const int f = blockIdx.x * CW + c;
-    const bool ok = f < 3 * np * g.KP;
-    const int cp = ok ? f / (np * g.KP) : 0, rem = ok ? f % (np * g.KP) : 0;
-    const int pi = rem / g.KP, k1c = rem % g.KP;
-    const int p = (a.traction && pi == a.nbody) ? g.sx3 : pi;
-    const size_t base = sidx(g, cp, p, 0, k1c);
-    float2 x[N1];
-#pragma unroll
-    for (int j1 = 0; j1 < N1; j1++)
-        x[j1] = ok ? a.S[base + (size_t)(N2 * j1 + t) * g.KP] : make_float2(0.f, 0.f);
-    RDft<N1, SIGN>::run(x);
-#pragma unroll
-    for (int k1 = 1; k1 < N1; k1++)
-        if (t) x[k1] = cmul(x[k1], twn<SIGN>(a.py.tw, t * k1));
-#pragma unroll
-    for (int k1 = 0; k1 < N1; k1++) smy[(k1 * N2 + t) * CW + c] = x[k1];
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-        float2 y[N2];
-        const int k1 = t + N2 * q;
-#pragma unroll
-        for (int jj = 0; jj < N2; jj++) y[jj] = smy[(k1 * N2 + jj) * CW + c];
-        RDft<N2, SIGN>::run(y);
-        if (ok) {
-#pragma unroll
-            for (int k2 = 0; k2 < N2; k2++) a.S[base + (size_t)(k1 + N1 * k2) * g.KP] = y[k2];
-        }
-    }
-    (void)n;
-}
-
 __global__ void __launch_bounds__(RELAX_NTHREADS) k_xinv(XiArgs a)
 {
     extern __shared__ float2 sm[];

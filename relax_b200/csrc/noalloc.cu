@@ -165,7 +165,7 @@ extern "C" int relax_op_green_noalloc(float *c1, float *c2, float *c3, float *t1
     xa.scale3 = (float)(dx1 * dx2 * dx3);
     xa.scale2 = (float)(dx1 * dx2);
     k_xfwd<XIN_REAL><<<dim3(sx2 / rows, sx3 + 1), RELAX_NTHREADS, smx, st>>>(xa);
-    YArgs ya{g, S, py, twy, sx3, 1};
+    YArgs ya{g, S, py, nullptr, twy, sx3, 1};
     k_ypass<-1><<<dim3((g.K1 + twy - 1) / twy, sx3 + 1, 3), RELAX_NTHREADS, smy, st>>>(ya);
     ZArgs za{};
     za.g = g; za.S = S; za.pz = pz; za.tw = twz; za.nin = sx3; za.nout = sx3;
@@ -173,7 +173,7 @@ extern "C" int relax_op_green_noalloc(float *c1, float *c2, float *c3, float *t1
     za.ratio2 = (float)(mu / (lambda + mu));
     za.lambda = lambda; za.mu = mu; za.gam = gam;
     k_zspec<<<dim3((g.K1 + twz - 1) / twz, sx2), RELAX_NTHREADS, smz, st>>>(za);
-    YArgs yb{g, S, py, twy, sx3, 0};
+    YArgs yb{g, S, py, nullptr, twy, sx3, 0};
     k_ypass<+1><<<dim3((g.K1 + twy - 1) / twy, sx3, 3), RELAX_NTHREADS, smy, st>>>(yb);
     XiArgs xi{};
     for (int k = 0; k < 3; k++) { xi.out[k] = cs[k]; xi.base[k] = nullptr; }

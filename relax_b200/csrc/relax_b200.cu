@@ -285,47 +285,6 @@ struct Prof {
         if (prof) (prof)->end(st);                          \
     } while (0)
 
-// register-resident column passes for the lengths they are instantiated for
-constexpr int kCW = 16;
-
-template <int N1, int N2, int SIGN>
-static void launch_ypass_sign(const YArgs &ya, dim3 grid, size_t sm, int nm, cudaStream_t st)
-{
-    if (nm > 1) {
-        set_smem(k_ypass_reg<N1, N2, kCW, SIGN, true>, sm);
-        launch_pdl(k_ypass_reg<N1, N2, kCW, SIGN, true>, dim3(grid.x, nm), kCW * N2, sm, st, ya);
-    } else {
-        set_smem(k_ypass_reg<N1, N2, kCW, SIGN>, sm);
-        launch_pdl(k_ypass_reg<N1, N2, kCW, SIGN>, grid, kCW * N2, sm, st, ya);
-    }
-}
-
-template <int N1, int N2>
-static cudaError_t launch_ypass_reg(const YArgs &ya, int sign, dim3 grid, int nm, cudaStream_t st)
-{
-    const size_t sm = (size_t)N1 * N2 * kCW * sizeof(float2);
-    if (sign < 0) launch_ypass_sign<N1, N2, -1>(ya, grid, sm, nm, st);
-    else launch_ypass_sign<N1, N2, +1>(ya, grid, sm, nm, st);
-    return cudaGetLastError();
-}
-
-static bool ypass_reg(const YArgs &ya, int sign, cudaStream_t st, cudaError_t *e, int nm = 1)
-{
-    // CW columns per block over the flattened (component, plane, k1) columns
-    const size_t ncol = (size_t)3 * (ya.nbody + ya.traction) * ya.g.KP;
-    const dim3 grid((unsigned)((ncol + kCW - 1) / kCW));
-    switch (ya.g.sx2) {
-    case 32: *e = launch_ypass_reg<8, 4>(ya, sign, grid, nm, st); return true;
-    case 96: *e = launch_ypass_reg<24, 4>(ya, sign, grid, nm, st); return true;
-    case 192: *e = launch_ypass_reg<24, 8>(ya, sign, grid, nm, st); return true;
-    case 64: *e = launch_ypass_reg<8, 8>(ya, sign, grid, nm, st); return true;
-    case 128: *e = launch_ypass_reg<16, 8>(ya, sign, grid, nm, st); return true;
-    case 256: *e = launch_ypass_reg<16, 16>(ya, sign, grid, nm, st); return true;
-    case 512: *e = launch_ypass_reg<32, 16>(ya, sign, grid, nm, st); return true;
-    default: return false;
-    }
-}
-
 template <int N1, int N2, int V>
 static void launch_xinv_v(const XiArgs &xi, int nout, size_t sm, int nm, cudaStream_t st)
 {
@@ -418,9 +377,7 @@ static bool xfwd_reg(const XfArgs &xa, bool div, int nplanes, cudaStream_t st, c
 static bool reg_shape(const Grid &g)
 {
     return (g.M == 32 || g.M == 64 || g.M == 96 || g.M == 128 || g.M == 256) && g.sx2 % 32 == 0 &&
-           (g.sx2 == 32 || g.sx2 == 64 || g.sx2 == 96 || g.sx2 == 128 || g.sx2 == 192 || g.sx2 == 256 ||
-            g.sx2 == 512) &&
-           zspec_batch_length(g.sx3);
+           ypass_batch_length(g.sx2) && zspec_batch_length(g.sx3);
 }
 
 // the x3 pass with its DFT-64 sub-transforms on the tensor cores: 128-deep
@@ -465,7 +422,7 @@ struct Spectral {
     float2 *S = nullptr;
     // in the buffer of S:
     float2 *tw = nullptr;          // tables for M, sx1, sx2, sx3
-    float4 *ptw = nullptr;         // those of sx3 as (cos, cos, sin, sin)
+    float4 *ptx = nullptr, *pty = nullptr, *ptz = nullptr;   // those of M, sx2, sx3 as (cos, cos, sin, sin)
     float4 *fg = nullptr;          // zspec_table for the planes that are written
     FftPlan pm{}, py{}, pz{};
     const float2 *tw1 = nullptr;
@@ -500,10 +457,10 @@ struct Spectral {
         const int ns[4] = {g.M, g.sx1, g.sx2, g.sx3};
         size_t tot = 0;
         for (int i = 0; i < 4; i++) tot += ns[i];
-        // one buffer: the spectrum, the correction table of the x3 pass, its
+        // one buffer: the spectrum, the correction table of the x3 pass, the
         // twiddles as (cos, cos, sin, sin) and the plain tables
         const size_t nrow = 3 * (size_t)(g.sx3 + 1) * g.sx2, nS = nrow * g.KP;
-        const size_t nfg = planes && zspec_length(g.sx3) ? 2 * zspec_table_stride(g) * planes : 0, np = 2 * (size_t)g.sx3;
+        const size_t nfg = planes && zspec_length(g.sx3) ? 2 * zspec_table_stride(g) * planes : 0, np = 2 * ((size_t)g.M + g.sx2 + g.sx3);
         std::vector<float2> h(np + tot);
         size_t off[4], o = 0;
         for (int i = 0; i < 4; i++) {
@@ -514,17 +471,21 @@ struct Spectral {
             }
             o += ns[i];
         }
-        for (int j = 0; j < g.sx3; j++) {
-            const float2 w = h[np + off[3] + j];
-            h[2 * j] = make_float2(w.x, w.x);
-            h[2 * j + 1] = make_float2(w.y, w.y);
-        }
+        size_t pos = 0;
+        for (int i : {0, 2, 3})
+            for (int j = 0; j < ns[i]; j++) {
+                const float2 w = h[np + off[i] + j];
+                h[pos++] = make_float2(w.x, w.x);
+                h[pos++] = make_float2(w.y, w.y);
+            }
         TRY(dalloc(&S, nS + nfg + h.size()));
         fg = nfg ? reinterpret_cast<float4 *>(S + nS) : nullptr;
-        ptw = reinterpret_cast<float4 *>(S + nS + nfg);
+        ptx = reinterpret_cast<float4 *>(S + nS + nfg);
+        pty = ptx + g.M;
+        ptz = pty + g.sx2;
         tw = S + nS + nfg + np;
         // (pageable memory: the call returns once the tables are staged)
-        CK(cudaMemcpyAsync(ptw, h.data(), h.size() * sizeof(float2), cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyAsync(ptx, h.data(), h.size() * sizeof(float2), cudaMemcpyHostToDevice, st));
         pm.tw = tw + off[0];
         tw1 = tw + off[1];
         py.tw = tw + off[2];
@@ -558,7 +519,7 @@ struct Spectral {
         if (ztab) dfree(ztab, idle);
         S = nullptr;
         tw = nullptr;
-        ptw = nullptr;
+        ptx = pty = ptz = nullptr;
         fg = nullptr;
         ztab = nullptr;
     }
@@ -572,11 +533,11 @@ struct Spectral {
         xa.scale2 = (float)(g.dx1 * g.dx2);
         return xa;
     }
-    YArgs yargs(int nplanes, int traction, int tile) const { return YArgs{g, S, py, tile, nplanes, traction}; }
+    YArgs yargs(int nplanes, int traction, int tile) const { return YArgs{g, S, py, pty, tile, nplanes, traction}; }
     ZArgs zargs(int nin, int nout, double lambda, double mu, double gam, int tile) const
     {
         ZArgs za{};
-        za.g = g; za.S = S; za.pz = pz; za.pt = ptw; za.tw = tile; za.nin = nin; za.nout = nout;
+        za.g = g; za.S = S; za.pz = pz; za.pt = ptz; za.tw = tile; za.nin = nin; za.nout = nout;
         za.ik1 = 1.0 / (g.sx1 * g.dx1); za.ik2 = 1.0 / (g.sx2 * g.dx2); za.ik3 = 1.0 / (g.sx3 * g.dx3);
         za.fg = fg; za.fgs = zspec_table_stride(g);
         za.ratio1 = (float)((lambda + mu) / (lambda + 2.0 * mu) / mu / (4.0 * M_PI * M_PI));
@@ -611,11 +572,10 @@ struct Spectral {
         YArgs ya = yargs(nin, 1, twy);
         cudaError_t re = cudaSuccess;
         if (use_reg) {
-            TIMED(prof, ST_YFWD, st, (ya.tw = kCW, yreg = ypass_reg(ya, -1, st, &re)));
+            TIMED(prof, ST_YFWD, st, (yreg = ypass_reg(ya, -1, st, &re)));
             if (re != cudaSuccess) return fail(RELAX_ERR_CUDA, "k_ypass_reg: %s", cudaGetErrorString(re));
         }
         if (!use_reg || !yreg) {
-            ya.tw = twy;
             TIMED(prof, ST_YFWD, st,
                   (k_ypass<-1><<<dim3((g.K1 + twy - 1) / twy, nin + 1, 3), RELAX_NTHREADS, smy, st>>>(ya)));
         }
@@ -637,12 +597,10 @@ struct Spectral {
         YArgs yb = yargs(nout, 0, twy);
         bool yr2 = false;
         if (use_reg) {
-            yb.tw = kCW;
             TIMED(prof, ST_YINV, st, (yr2 = ypass_reg(yb, +1, st, &re)));
             if (re != cudaSuccess) return fail(RELAX_ERR_CUDA, "k_ypass_reg: %s", cudaGetErrorString(re));
         }
         if (!yr2) {
-            yb.tw = twy;
             TIMED(prof, ST_YINV, st,
                   (k_ypass<+1><<<dim3((g.K1 + twy - 1) / twy, nout, 3), RELAX_NTHREADS, smy, st>>>(yb)));
         }
@@ -3286,14 +3244,14 @@ extern "C" int relax_op_fft3(float *data, int sx1, int sx2, int sx3, double dx1,
         // only component 0 is meaningful: point the others at the same data
         xa.in[1] = data; xa.in[2] = data;
         k_xfwd<XIN_REAL><<<dim3(sx2 / sp.rows, sx3), RELAX_NTHREADS, sp.smx, st>>>(xa);
-        YArgs ya{g, sp.S, sp.py, sp.twy, sx3, 0};
+        YArgs ya = sp.yargs(sx3, 0, sp.twy);
         k_ypass<-1><<<dim3((g.K1 + sp.twy - 1) / sp.twy, sx3, 1), RELAX_NTHREADS, sp.smy, st>>>(ya);
         k_zfft_plain<<<dim3((g.K1 + tw - 1) / tw, sx2), RELAX_NTHREADS, smz, st>>>(g, sp.S, sp.pz, tw, -1);
         k_spec_copy<<<nblocks((size_t)g.K1 * sx2 * sx3), RELAX_NTHREADS, 0, st>>>(g, sp.S, data, 1);
     } else {
         k_spec_copy<<<nblocks((size_t)g.K1 * sx2 * sx3), RELAX_NTHREADS, 0, st>>>(g, sp.S, data, 0);
         k_zfft_plain<<<dim3((g.K1 + tw - 1) / tw, sx2), RELAX_NTHREADS, smz, st>>>(g, sp.S, sp.pz, tw, +1);
-        YArgs yb{g, sp.S, sp.py, sp.twy, sx3, 0};
+        YArgs yb = sp.yargs(sx3, 0, sp.twy);
         k_ypass<+1><<<dim3((g.K1 + sp.twy - 1) / sp.twy, sx3, 1), RELAX_NTHREADS, sp.smy, st>>>(yb);
         // component 0 only: k_xinv handles 3 components; use a 1-row-per-line
         // variant through the same kernel with out/base of components 1,2
@@ -3557,9 +3515,9 @@ static int build_tables(relax_batch *b)
         corr[k] = stress_args(c, c->vp);
         end[k] = stress_args(c, c->u);
         xf[k] = c->sp.xargs(xf_div(c), g.sx3h);
-        yf[k] = c->sp.yargs(g.sx3h, 1, kCW);
-        yi[k] = c->sp.yargs(g.sx3h, 0, kCW);
-        z[k] = c->sp.zargs(g.sx3h, g.sx3h, c->cfg.lambda, c->cfg.mu, c->cfg.gam, kCW);
+        yf[k] = c->sp.yargs(g.sx3h, 1, 0);
+        yi[k] = c->sp.yargs(g.sx3h, 0, 0);
+        z[k] = c->sp.zargs(g.sx3h, g.sx3h, c->cfg.lambda, c->cfg.mu, c->cfg.gam, 0);
         xip[k] = c->sp.xiargs(xi_update(c, c->vp, c->u, 0.5f, true));
         xic[k] = c->sp.xiargs(xi_update(c, c->u, c->u, 1.0f, true));
         int tot = 0;

@@ -50,6 +50,7 @@ struct YArgs {
     Grid g;
     float2 *S;
     FftPlan py;
+    const float4 *pt;  // py.tw as (cos, cos, sin, sin)
     int tw;            // tile width (k1 columns)
     int nbody;         // body planes [0, nbody)
     int traction;      // also the traction plane (index nbody of blockIdx.y)
@@ -91,6 +92,7 @@ struct XiArgs {
 // The register-resident passes: false when the grid's length has no
 // instantiation (the caller takes the general kernel).  nm > 1: one launch
 // for the nm members of a batch, whose arguments are args.tab.
+bool ypass_reg(const YArgs &ya, int sign, cudaStream_t st, cudaError_t *e, int nm = 1);
 bool zspec_reg(const ZArgs &za, cudaStream_t st, cudaError_t *e, int nm = 1);
 // whether the x3 pass is instantiated for a length
 bool zspec_length(int sx3);
@@ -98,7 +100,8 @@ bool zspec_length(int sx3);
 // contents.  It depends on the grid alone.
 size_t zspec_table_stride(const Grid &g);
 cudaError_t zspec_table(const Grid &g, float4 *fg, int planes, cudaStream_t st);
-// lengths with batched instantiations of the x3 pass
+// lengths with batched instantiations
+bool ypass_batch_length(int sx2);
 bool zspec_batch_length(int sx3);
 
 }  // namespace relax

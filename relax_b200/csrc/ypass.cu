@@ -1,0 +1,152 @@
+// ypass.cu -- transforms of the spectrum along x2.
+#include "launch.cuh"
+#include "pfft.cuh"
+#include "spectral.cuh"
+
+namespace relax {
+namespace {
+
+constexpr int CW = 8;   // column pairs of a block: 128-byte segments
+
+// blocks on an SM: what shared memory holds, but no more than leave a thread
+// 90 registers beside its largest group.  With 40 the transforms spill: 223
+// instead of 176 us a pass on the 512 x 512 x 256 box, 14 instead of 11.5 us
+// on 128^3.
+constexpr int yblocks(int N1, int N2)
+{
+    const int sm = 233472 / (N1 * N2 * CW * 16 + 1024);
+    const int rg = 65536 / ((4 * (N1 > N2 ? N1 : N2) + 90) * ((CW * N2 + 31) / 32 * 32));
+    const int m = sm < rg ? sm : rg;
+    return m < 1 ? 1 : m > 16 ? 16 : m;
+}
+
+// Passes 2 and 4: the spectrum's columns (component, plane, x1 wavenumber)
+// along x2, two neighbouring ones per thread (pfft.cuh), N2 threads a pair,
+// one exchange through shared memory.  Half the instructions of one column
+// per thread (5.9 instead of 11 M warp instructions on the 256 x 256 x 128
+// box), so what bounds it is the latency of the loads: 27.7 -> 26.4 us
+// forward and 25.8 -> 22.6 us inverse there, 187 -> 176 us on 512 x 512 x
+// 256; 84 -> 29 us on 288 x 216 x 144 against the general kernel.
+template <int N1, int N2, int SIGN, bool BATCH>
+__global__ void __launch_bounds__(CW *N2, yblocks(N1, N2)) k_ypass_p(const __grid_constant__ YArgs a0)
+{
+    pdl_enter();
+    const YArgs &a = BATCH ? a0.tab[blockIdx.y] : a0;
+    constexpr int n = N1 * N2, Q = (N1 + N2 - 1) / N2, IM = n * CW;
+    static_assert(N1 >= N2, "shape");
+    extern __shared__ float2 U[];   // real parts [N1][N2][CW], imaginary parts
+    const Grid &g = a.g;
+    const int c = threadIdx.x % CW, t = threadIdx.x / CW;
+    const int KP2 = g.KP / 2, np = a.nbody + a.traction;
+    // pairs flattened: f = (cp np + pi) KP2 + kk
+    const int f = blockIdx.x * CW + c;
+    const bool ok = f < 3 * np * KP2;
+    const int cpi = ok ? f / KP2 : 0, cp = cpi / np, pi = cpi - cp * np;
+    const int p = (a.traction && pi == a.nbody) ? g.sx3 : pi;
+    float4 *S = reinterpret_cast<float4 *>(a.S + sidx(g, cp, p, 0, 0)) + (ok ? f - cpi * KP2 : 0);
+    // 8-byte accesses of a half-warp are two runs of CW pairs: the swizzle
+    // puts rows k1 and k1 + 1 into different halves of the banks (for odd N2
+    // they are there already)
+    auto uidx = [&](int k1, int j) { return (k1 * N2 + (N2 % 2 ? j : j ^ (k1 & 1))) * CW + c; };
+    {
+        P2 x[N1];
+#pragma unroll
+        for (int j1 = 0; j1 < N1; j1++) x[j1] = pair(S[(N2 * j1 + t) * KP2]);
+        PDft<N1, SIGN>::run(x);
+#pragma unroll
+        for (int k1 = 0; k1 < N1; k1++) {
+            const P2 v = k1 ? pmul<(SIGN > 0)>(x[k1], w2(__ldg(a.pt + t * k1))) : x[k1];
+            const int q = uidx(k1, t);
+            U[q] = v.r;
+            U[q + IM] = v.i;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+        const int k1 = t + N2 * q;
+        if (N1 % N2 && k1 >= N1) break;
+        P2 y[N2];
+#pragma unroll
+        for (int jj = 0; jj < N2; jj++) {
+            const int u = uidx(k1, jj);
+            y[jj] = {U[u], U[u + IM]};
+        }
+        PDft<N2, SIGN>::run(y);
+        if (ok) {
+#pragma unroll
+            for (int k2 = 0; k2 < N2; k2++) S[(k1 + N1 * k2) * KP2] = unpair(y[k2]);
+        }
+    }
+}
+
+template <int N1, int N2, bool BATCH>
+void launch(const YArgs &ya, int sign, int nm, cudaStream_t st)
+{
+    const size_t sm = (size_t)N1 * N2 * CW * 16;
+    const size_t np = (size_t)3 * (ya.nbody + ya.traction) * (ya.g.KP / 2);
+    const dim3 grid((unsigned)((np + CW - 1) / CW), nm);
+    auto run = [&](void (*k)(YArgs)) {
+        set_smem(k, sm);
+        launch_pdl(k, grid, CW * N2, sm, st, ya);
+    };
+    if (sign < 0) run(k_ypass_p<N1, N2, -1, BATCH>);
+    else run(k_ypass_p<N1, N2, +1, BATCH>);
+}
+
+}  // namespace
+
+bool ypass_batch_length(int n)
+{
+    return n == 32 || n == 64 || n == 96 || n == 128 || n == 192 || n == 256 || n == 512;
+}
+
+// The products of 2 and 3 from 24 to 512; other lengths take k_ypass.
+bool ypass_reg(const YArgs &ya, int sign, cudaStream_t st, cudaError_t *e, int nm)
+{
+    if (nm > 1) {
+        switch (ya.g.sx2) {
+        case 32: launch<8, 4, true>(ya, sign, nm, st); break;
+        case 64: launch<8, 8, true>(ya, sign, nm, st); break;
+        case 96: launch<12, 8, true>(ya, sign, nm, st); break;
+        case 128: launch<16, 8, true>(ya, sign, nm, st); break;
+        case 192: launch<24, 8, true>(ya, sign, nm, st); break;
+        case 256: launch<16, 16, true>(ya, sign, nm, st); break;
+        case 512: launch<32, 16, true>(ya, sign, nm, st); break;
+        default: return false;
+        }
+        *e = cudaGetLastError();
+        return true;
+    }
+    switch (ya.g.sx2) {
+    case 24: launch<6, 4, false>(ya, sign, nm, st); break;
+    case 27: launch<9, 3, false>(ya, sign, nm, st); break;
+    case 32: launch<8, 4, false>(ya, sign, nm, st); break;
+    case 36: launch<6, 6, false>(ya, sign, nm, st); break;
+    case 48: launch<12, 4, false>(ya, sign, nm, st); break;
+    case 54: launch<9, 6, false>(ya, sign, nm, st); break;
+    case 64: launch<8, 8, false>(ya, sign, nm, st); break;
+    case 72: launch<12, 6, false>(ya, sign, nm, st); break;
+    case 81: launch<9, 9, false>(ya, sign, nm, st); break;
+    case 96: launch<12, 8, false>(ya, sign, nm, st); break;
+    case 108: launch<18, 6, false>(ya, sign, nm, st); break;
+    case 128: launch<16, 8, false>(ya, sign, nm, st); break;
+    case 144: launch<12, 12, false>(ya, sign, nm, st); break;
+    case 162: launch<18, 9, false>(ya, sign, nm, st); break;
+    case 192: launch<24, 8, false>(ya, sign, nm, st); break;
+    case 216: launch<24, 9, false>(ya, sign, nm, st); break;
+    case 243: launch<27, 9, false>(ya, sign, nm, st); break;
+    case 256: launch<16, 16, false>(ya, sign, nm, st); break;
+    case 288: launch<24, 12, false>(ya, sign, nm, st); break;
+    case 324: launch<18, 18, false>(ya, sign, nm, st); break;
+    case 384: launch<24, 16, false>(ya, sign, nm, st); break;
+    case 432: launch<24, 18, false>(ya, sign, nm, st); break;
+    case 486: launch<27, 18, false>(ya, sign, nm, st); break;
+    case 512: launch<32, 16, false>(ya, sign, nm, st); break;
+    default: return false;
+    }
+    *e = cudaGetLastError();
+    return true;
+}
+
+}  // namespace relax

@@ -22,6 +22,7 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 X3 = (24, 32, 36, 48, 54, 64, 72, 96, 108, 128, 144, 162, 192, 216, 256, 288, 384, 512)
+X2 = (24, 27, 32, 36, 48, 54, 64, 72, 81, 96, 108, 128, 144, 162, 192, 216, 243, 256, 288, 324, 384, 432, 486, 512)
 
 
 def green_error(oracle, sx1, sx2, sx3, gam=8.3e-4):
@@ -59,3 +60,8 @@ def test_x3_lengths(oracle32, sx3):
     assert green_error(oracle32, 24, 27, sx3) < 1e-5     # odd sx2: the wavenumbers are not symmetric
     errs = step_errors(oracle32, 24, 18, sx3)
     assert max(errs.values()) < 1e-5, errs
+
+
+@pytest.mark.parametrize("sx2", X2)
+def test_x2_lengths(oracle32, sx2):
+    assert green_error(oracle32, 24, sx2, 32) < 1e-5
