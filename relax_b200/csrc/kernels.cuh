@@ -1172,151 +1172,6 @@ __global__ void __launch_bounds__(RELAX_NTHREADS) k_xfwd(XfArgs a)
 }
 
 
-// pass 1, register-resident: -div(m) (or the traction m_i3, or real input
-// rows) -> packed real FFT along x1 for rows of M = N1*N2 complex values; RW
-// rows of one plane per block, N2 threads per row, components in turn.
-// The body force of the block's rows is first built in the row buffers with
-// float4 loads (x neighbours by warp shuffle, one wrap-around load per warp
-// edge), then each row thread picks its stride-N2 elements from there.
-template <int XIN, int N1, int N2, int RW, bool BATCH = false>
-__global__ void __launch_bounds__(RW *N2, (RW * N2 <= 128) ? 8 : 4) k_xfwd_reg(const __grid_constant__ XfArgs a0)
-{
-    pdl_enter();
-    const XfArgs &a = BATCH ? a0.tab[blockIdx.z] : a0;
-    constexpr int M = N1 * N2, Q = N1 / N2, N2P = N2 + 1, NT = RW * N2;
-    constexpr int RS0 = (N1 * N2P > M + 1 ? N1 * N2P : M + 1);
-    constexpr int RS = RS0 + ((8 - RS0 % 16) + 16) % 16;
-    constexpr int SX1 = 2 * M, R4 = SX1 / 4, ITS = RW * R4 / NT;
-    static_assert(N1 % N2 == 0, "N1 must be a multiple of N2");
-    static_assert(NT % 32 == 0 && (RW * R4) % NT == 0, "rows split evenly over the block");
-    // x neighbours by shuffle when every warp stages part of one row
-    constexpr bool SHFL = R4 % 32 == 0;
-    static_assert(RS % 2 == 0, "row buffers start on 16 bytes");
-    extern __shared__ float2 smx[];
-    const Grid &g = a.g;
-    const int t = threadIdx.x % N2, r = threadIdx.x / N2, lane = threadIdx.x & 31;
-    const int i2 = blockIdx.x * RW + r, pi = blockIdx.y;
-    const bool trac = a.has_trac && pi == a.nin;
-    const int i3 = pi;
-    float2 *T = smx + r * RS;
-    const size_t rowo = (size_t)i2 * g.sx1;
-#pragma unroll 1
-    for (int c = 0; c < 3; c++) {
-        float2 z[N1];
-        if (XIN == XIN_DIV && !trac) {
-            const int cx = c == 0 ? 0 : c == 1 ? 1 : 2;
-            const int cy = c == 0 ? 1 : c == 1 ? 3 : 4;
-            const int cz = c == 0 ? 2 : c == 1 ? 4 : 5;
-            const size_t pl = (size_t)i3 * g.plane;
-            size_t zp, zm;
-            float kz;
-            if (i3 == 0) { zp = g.plane; zm = 0; kz = a.k3b; }
-            else if (i3 == g.sx3h - 1) { zp = pl; zm = pl - g.plane; kz = a.k3b; }
-            else { zp = pl + g.plane; zm = pl - g.plane; kz = a.k3; }
-#pragma unroll 4
-            for (int it = 0; it < ITS; it++) {
-                const int q = threadIdx.x + NT * it, rr = q / R4, x = 4 * (q % R4);
-                const int row = blockIdx.x * RW + rr;
-                const float *mx = a.m + cx * g.nh + pl + (size_t)row * SX1;
-                const float4 xc = __ldg(reinterpret_cast<const float4 *>(mx + x));
-                float xl, xr;
-                if (SHFL) {
-                    xl = __shfl_up_sync(0xffffffffu, xc.w, 1);
-                    xr = __shfl_down_sync(0xffffffffu, xc.x, 1);
-                    if (lane == 0) xl = __ldg(mx + (x + SX1 - 1) % SX1);
-                    if (lane == 31) xr = __ldg(mx + (x + 4) % SX1);
-                } else {
-                    xl = __ldg(mx + (x + SX1 - 1) % SX1);
-                    xr = __ldg(mx + (x + 4) % SX1);
-                }
-                const float *my = a.m + cy * g.nh + pl + x;
-                const float4 yp = __ldg(reinterpret_cast<const float4 *>(my + (size_t)((row + 1) % g.sx2) * SX1));
-                const float4 ym =
-                    __ldg(reinterpret_cast<const float4 *>(my + (size_t)((row + g.sx2 - 1) % g.sx2) * SX1));
-                const float *mz = a.m + cz * g.nh + (size_t)row * SX1 + x;
-                const float4 zpv = __ldg(reinterpret_cast<const float4 *>(mz + zp));
-                const float4 zmv = __ldg(reinterpret_cast<const float4 *>(mz + zm));
-                float4 f;
-                f.x = -((xc.y - xl) * a.k1 + (yp.x - ym.x) * a.k2 + (zpv.x - zmv.x) * kz) * a.scale3;
-                f.y = -((xc.z - xc.x) * a.k1 + (yp.y - ym.y) * a.k2 + (zpv.y - zmv.y) * kz) * a.scale3;
-                f.z = -((xc.w - xc.y) * a.k1 + (yp.z - ym.z) * a.k2 + (zpv.z - zmv.z) * kz) * a.scale3;
-                f.w = -((xr - xc.z) * a.k1 + (yp.w - ym.w) * a.k2 + (zpv.w - zmv.w) * kz) * a.scale3;
-                *reinterpret_cast<float4 *>(reinterpret_cast<float *>(smx + rr * RS) + x) = f;
-            }
-            __syncthreads();
-#pragma unroll
-            for (int j1 = 0; j1 < N1; j1++) z[j1] = T[N2 * j1 + t];
-            __syncthreads();
-        } else if (XIN == XIN_DIV) {
-            const int cz = c == 0 ? 2 : c == 1 ? 4 : 5;
-            {
-                const float *mt = a.m + cz * g.nh + rowo;
-#pragma unroll
-                for (int j1 = 0; j1 < N1; j1++) {
-                    const int i1 = 2 * (N2 * j1 + t);
-                    float2 v = *reinterpret_cast<const float2 *>(mt + i1);
-                    if (c == 2 && a.tload) {
-                        const float2 l = *reinterpret_cast<const float2 *>(a.tload + rowo + i1);
-                        v.x += l.x; v.y += l.y;
-                    }
-                    z[j1] = make_float2(v.x * a.scale2, v.y * a.scale2);
-                }
-            }
-        } else {
-#pragma unroll
-            for (int j1 = 0; j1 < N1; j1++) {
-                const int i1 = 2 * (N2 * j1 + t);
-                float2 v;
-                if (trac) {
-                    v = make_float2(a.tin[c][(size_t)i2 * a.trp + i1], a.tin[c][(size_t)i2 * a.trp + i1 + 1]);
-                    if (c == 2 && a.tload) { v.x += a.tload[rowo + i1]; v.y += a.tload[rowo + i1 + 1]; }
-                    v.x *= a.scale2; v.y *= a.scale2;
-                } else {
-                    const float *src = a.in[c] + (size_t)i3 * a.pp + (size_t)i2 * a.rp + i1;
-                    v = make_float2(src[0] * a.scale3, src[1] * a.scale3);
-                }
-                z[j1] = v;
-            }
-        }
-        // complex FFT of length M of the packed row
-        RDft<N1, -1>::run(z);
-#pragma unroll
-        for (int k1 = 1; k1 < N1; k1++)
-            if (t) z[k1] = cmul(z[k1], twn<-1>(a.pm.tw, t * k1));
-#pragma unroll
-        for (int k1 = 0; k1 < N1; k1++) T[k1 * N2P + t] = z[k1];
-        __syncthreads();
-        float2 y[Q][N2];
-#pragma unroll
-        for (int q = 0; q < Q; q++) {
-#pragma unroll
-            for (int jj = 0; jj < N2; jj++) y[q][jj] = T[(t + N2 * q) * N2P + jj];
-            RDft<N2, -1>::run(y[q]);
-        }
-        __syncthreads();
-        // natural order Z[k1 + N1 k2] into the row buffer for the unpacking
-#pragma unroll
-        for (int q = 0; q < Q; q++)
-#pragma unroll
-            for (int k2 = 0; k2 < N2; k2++) T[(t + N2 * q) + N1 * k2] = y[q][k2];
-        __syncthreads();
-        const int p = trac ? g.sx3 : i3;
-        float2 *dst = a.S + sidx(g, c, p, i2, 0);
-        for (int k = t; k <= M; k += N2) {
-            const float2 zk = T[k == M ? 0 : k];
-            const float2 zm = cconj(T[k == 0 ? 0 : M - k]);
-            const float2 e = cscale(cadd(zk, zm), 0.5f);
-            const float2 d = csub(zk, zm);
-            const float2 w = __ldg(&a.tw1[k]);
-            const float2 wd = cmul(w, d);
-            dst[k] = make_float2(e.x + 0.5f * wd.y, e.y - 0.5f * wd.x);
-        }
-        __syncthreads();
-    }
-}
-
-
-
 template <int SIGN>
 __global__ void __launch_bounds__(RELAX_NTHREADS) k_ypass(YArgs a)
 {

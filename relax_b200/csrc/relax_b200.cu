@@ -332,51 +332,10 @@ static bool xinv_reg(const XiArgs &xi, int nout, cudaStream_t st, cudaError_t *e
     }
 }
 
-template <int XIN, int N1, int N2>
-static void launch_xfwd_in(const XfArgs &xa, dim3 grid, size_t sm, int nm, cudaStream_t st)
-{
-    constexpr int RW = 16;
-    if (nm > 1) {
-        set_smem(k_xfwd_reg<XIN, N1, N2, RW, true>, sm);
-        launch_pdl(k_xfwd_reg<XIN, N1, N2, RW, true>, dim3(grid.x, grid.y, nm), RW * N2, sm, st, xa);
-    } else {
-        set_smem(k_xfwd_reg<XIN, N1, N2, RW>, sm);
-        launch_pdl(k_xfwd_reg<XIN, N1, N2, RW>, grid, RW * N2, sm, st, xa);
-    }
-}
-
-template <int N1, int N2>
-static cudaError_t launch_xfwd_reg(const XfArgs &xa, bool div, dim3 grid, int nm, cudaStream_t st)
-{
-    constexpr int RW = 16, N2P = N2 + 1, M = N1 * N2;
-    constexpr int RS0 = (N1 * N2P > M + 1 ? N1 * N2P : M + 1), RS = RS0 + ((8 - RS0 % 16) + 16) % 16;
-    const size_t sm = (size_t)RW * RS * sizeof(float2);
-    if (div) launch_xfwd_in<XIN_DIV, N1, N2>(xa, grid, sm, nm, st);
-    else launch_xfwd_in<XIN_REAL, N1, N2>(xa, grid, sm, nm, st);
-    return cudaGetLastError();
-}
-
-static bool xfwd_reg(const XfArgs &xa, bool div, int nplanes, cudaStream_t st, cudaError_t *e, int nm = 1)
-{
-    // the 7-point filters are applied by k_xfwd alone (grids of the x2
-    // filter have no rows of 16 anyway, nor those of the x1 filter a register
-    // x pass)
-    if (xa.g.sx2 % 16 || (div && (xa.fx.n || xa.fy.n))) return false;
-    const dim3 grid(xa.g.sx2 / 16, nplanes);
-    switch (xa.g.M) {
-    case 32: *e = launch_xfwd_reg<8, 4>(xa, div, grid, nm, st); return true;
-    case 96: *e = launch_xfwd_reg<24, 4>(xa, div, grid, nm, st); return true;
-    case 64: *e = launch_xfwd_reg<8, 8>(xa, div, grid, nm, st); return true;
-    case 128: *e = launch_xfwd_reg<16, 8>(xa, div, grid, nm, st); return true;
-    case 256: *e = launch_xfwd_reg<16, 16>(xa, div, grid, nm, st); return true;
-    default: return false;
-    }
-}
-
 // the lengths the register passes are instantiated for
 static bool reg_shape(const Grid &g)
 {
-    return (g.M == 32 || g.M == 64 || g.M == 96 || g.M == 128 || g.M == 256) && g.sx2 % 32 == 0 &&
+    return xpass_batch_length(g.M) && g.sx2 % 32 == 0 &&
            ypass_batch_length(g.sx2) && zspec_batch_length(g.sx3);
 }
 
@@ -528,7 +487,7 @@ struct Spectral {
     // kept: the input / epilogue fields)
     XfArgs xargs(XfArgs xa, int nin) const
     {
-        xa.g = g; xa.S = S; xa.pm = pm; xa.tw1 = tw1; xa.nin = nin; xa.rows = rows; xa.has_trac = 1;
+        xa.g = g; xa.S = S; xa.pm = pm; xa.pt = ptx; xa.tw1 = tw1; xa.nin = nin; xa.rows = rows; xa.has_trac = 1;
         xa.scale3 = (float)(g.dx1 * g.dx2 * g.dx3);
         xa.scale2 = (float)(g.dx1 * g.dx2);
         return xa;
@@ -547,7 +506,7 @@ struct Spectral {
     }
     XiArgs xiargs(XiArgs xi) const
     {
-        xi.g = g; xi.S = S; xi.pm = pm; xi.tw1 = tw1; xi.rows = rows;
+        xi.g = g; xi.S = S; xi.pm = pm; xi.pt = ptx; xi.tw1 = tw1; xi.rows = rows;
         xi.scale = (float)(2.0 / ((double)g.sx1 * g.dx1 * g.sx2 * g.dx2 * g.sx3 * g.dx3));
         return xi;
     }
@@ -562,7 +521,7 @@ struct Spectral {
         bool xr0 = false;
         cudaError_t re0 = cudaSuccess;
         if (use_reg) {
-            TIMED(prof, ST_XFWD, st, (xr0 = xfwd_reg(xa, div, nin + 1, st, &re0)));
+            TIMED(prof, ST_XFWD, st, (xr0 = xfwd_reg(xa, div, st, &re0)));
             if (re0 != cudaSuccess) return fail(RELAX_ERR_CUDA, "k_xfwd_reg: %s", cudaGetErrorString(re0));
         }
         if (!xr0) {
@@ -3602,7 +3561,7 @@ static int batch_green(relax_batch *b, const XiArgs &xi0)
     const int n = (int)b->m.size();
     const Grid &g = b->m[0]->g;
     cudaError_t e = cudaSuccess;
-    if (!xfwd_reg(t.xf0, true, g.sx3h + 1, b->st, &e, n) || e != cudaSuccess)
+    if (!xfwd_reg(t.xf0, true, b->st, &e, n) || e != cudaSuccess)
         return fail(RELAX_ERR_CUDA, "batched x pass: %s", cudaGetErrorString(e));
     if (!ypass_reg(t.yf0, -1, b->st, &e, n) || e != cudaSuccess)
         return fail(RELAX_ERR_CUDA, "batched y pass: %s", cudaGetErrorString(e));

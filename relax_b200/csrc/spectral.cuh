@@ -30,6 +30,7 @@ struct XfArgs {
     Grid g;
     float2 *S;
     FftPlan pm;              // complex length M = sx1/2
+    const float4 *pt;        // pm.tw as (cos, cos, sin, sin)
     const float2 *tw1;       // exp(-2 pi i k / sx1)
     int nin, rows;
     int has_trac;            // blockIdx.y == nin is the traction plane
@@ -42,7 +43,7 @@ struct XfArgs {
     size_t trp;
     const float *tload;      // optional surface load added to t3 (sx1 x sx2)
     float scale3, scale2;
-    const struct XfArgs *tab;   // batched launch: one entry per member (blockIdx.z)
+    const struct XfArgs *tab;   // batched launch: one entry per member (blockIdx.y)
 };
 
 // pass 2 / 4: complex transform along x2 for a tile of x1 wavenumbers
@@ -77,6 +78,7 @@ struct XiArgs {
     Grid g;
     const float2 *S;
     FftPlan pm;
+    const float4 *pt;
     const float2 *tw1;
     int rows;
     float *out[3];
@@ -92,6 +94,7 @@ struct XiArgs {
 // The register-resident passes: false when the grid's length has no
 // instantiation (the caller takes the general kernel).  nm > 1: one launch
 // for the nm members of a batch, whose arguments are args.tab.
+bool xfwd_reg(const XfArgs &xa, bool div, cudaStream_t st, cudaError_t *e, int nm = 1);
 bool ypass_reg(const YArgs &ya, int sign, cudaStream_t st, cudaError_t *e, int nm = 1);
 bool zspec_reg(const ZArgs &za, cudaStream_t st, cudaError_t *e, int nm = 1);
 // whether the x3 pass is instantiated for a length
@@ -101,6 +104,7 @@ bool zspec_length(int sx3);
 size_t zspec_table_stride(const Grid &g);
 cudaError_t zspec_table(const Grid &g, float4 *fg, int planes, cudaStream_t st);
 // lengths with batched instantiations
+bool xpass_batch_length(int M);
 bool ypass_batch_length(int sx2);
 bool zspec_batch_length(int sx3);
 

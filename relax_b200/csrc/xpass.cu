@@ -1,0 +1,306 @@
+// xpass.cu -- the real transforms along x1: forward with the body force of
+// the moment tensor, inverse with the field update.
+//
+// A row of sx1 = 2 M real values is a complex transform of length M = N1 N2
+// of its neighbouring pairs (x[2j], x[2j+1]).  Two neighbouring rows go
+// together through f32x2 instructions (pfft.cuh), N2 threads per pair of
+// rows, one shared-memory exchange inside the transform and one on either
+// side of it; real and imaginary parts (of two rows: 8 bytes) are in separate
+// arrays.  Pairs of rows are numbered through all planes, so that no block
+// is left partly empty at a plane's end.
+#include <cuda_bf16.h>
+
+#include "launch.cuh"
+#include "pfft.cuh"
+#include "spectral.cuh"
+
+namespace relax {
+namespace {
+
+// row pairs of a block, for about 64 threads (with 128 the last wave costs
+// more: 55.5 instead of 52.5 us forward on the 256 x 256 x 128 box)
+__host__ __device__ constexpr int xpairs(int N2) { return 64 / N2; }
+// row pitch in shared memory: the longer of the row and its padded transpose
+// [N1][N2 | 1], and N2 more than a multiple of 16, so that the N2 threads of
+// neighbouring rows reach different banks
+__host__ __device__ constexpr int xpitch(int N1, int N2)
+{
+    const int n = N1 * (N2 | 1);
+    return n + ((N2 - n) % 16 + 16) % 16;
+}
+__host__ __device__ constexpr size_t xsmem(int N1, int N2)
+{
+    return (size_t)xpairs(N2) * (xpitch(N1, N2) * 16 + sizeof(int2));
+}
+constexpr int xblocks(int N1, int N2, int extra)
+{
+    const int sm = (int)(233472 / (xsmem(N1, N2) + 1024));
+    const int rg = 65536 / ((4 * (N1 > N2 ? N1 : N2) + extra) * ((xpairs(N2) * N2 + 31) / 32 * 32));
+    const int m = sm < rg ? sm : rg;
+    return m < 1 ? 1 : m > 16 ? 16 : m;
+}
+
+// complex transform of the block's row pairs, from T (natural order) to T
+// (natural order); every thread has one pair's t, those beyond the last pair none
+template <int N1, int N2, int SIGN>
+__device__ __forceinline__ void row_fft(float2 *T, int IM, int t, bool on, const float4 *pt)
+{
+    constexpr int Q = (N1 + N2 - 1) / N2, NP = N2 | 1;
+    P2 z[N1];
+    if (on) {
+#pragma unroll
+        for (int j1 = 0; j1 < N1; j1++) z[j1] = {T[N2 * j1 + t], T[N2 * j1 + t + IM]};
+    }
+    __syncthreads();
+    if (on) {
+        PDft<N1, SIGN>::run(z);
+#pragma unroll
+        for (int k1 = 0; k1 < N1; k1++) {
+            const P2 v = k1 ? pmul<(SIGN > 0)>(z[k1], w2(__ldg(pt + t * k1))) : z[k1];
+            T[k1 * NP + t] = v.r;
+            T[k1 * NP + t + IM] = v.i;
+        }
+    }
+    __syncthreads();
+    P2 y[Q][N2];
+    if (on) {
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+            const int k1 = t + N2 * q;
+            if (N1 % N2 && k1 >= N1) break;
+#pragma unroll
+            for (int jj = 0; jj < N2; jj++) y[q][jj] = {T[k1 * NP + jj], T[k1 * NP + jj + IM]};
+            PDft<N2, SIGN>::run(y[q]);
+        }
+    }
+    __syncthreads();
+    if (on) {
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+            const int k1 = t + N2 * q;
+            if (N1 % N2 && k1 >= N1) break;
+#pragma unroll
+            for (int k2 = 0; k2 < N2; k2++) {
+                T[k1 + N1 * k2] = y[q][k2].r;
+                T[k1 + N1 * k2 + IM] = y[q][k2].i;
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// Pass 1: -div(m) of the moment tensor (equivalentbodyforce,
+// src/elastic3d.f90:1214-1506; central differences) or real input rows, and
+// the surface traction, through the R2C transform along x1 into the spectrum.
+// A block takes one component (the fastest block index, so that the blocks
+// that share moment components run together).  The planes go from the last
+// to the first: the stress pass before has just written the last ones, which
+// are in L2 still (53.2 -> 48.5 us on the 256 x 256 x 128 box).  What bounds
+// the pass is the latency of its 10 loads per two groups of 4 points:
+// 52.3 -> 48.5 us on that box against one row per thread, 346 -> 320 us on
+// 512 x 512 x 256, 20.4 -> 16.4 us on 128^3; 187 -> 56 us on 288 x 216 x 144
+// against the general kernel.
+template <int XIN, int N1, int N2, bool BATCH>
+__global__ void __launch_bounds__(xpairs(N2) *N2, xblocks(N1, N2, 60)) k_xfwd_p(const __grid_constant__ XfArgs a0)
+{
+    pdl_enter();
+    const XfArgs &a = BATCH ? a0.tab[blockIdx.y] : a0;
+    constexpr int M = N1 * N2, SX1 = 2 * M, R4 = SX1 / 4, RP = xpairs(N2), NT = RP * N2, RS = xpitch(N1, N2);
+    constexpr int IM = RP * RS;
+    static_assert(M % 2 == 0, "rows of whole float4");
+    extern __shared__ __align__(16) float2 sm[];
+    const Grid &g = a.g;
+    const int c = blockIdx.x % 3, f0 = (gridDim.x / 3 - 1 - blockIdx.x / 3) * RP;   // the last planes first
+    const int npr = (g.sx2 + 1) / 2, F = (a.nin + 1) * npr;   // the last plane is the traction's
+    const int cx = c, cy = c == 0 ? 1 : c == 1 ? 3 : 4, cz = c == 0 ? 2 : c == 1 ? 4 : 5;
+    // the halves of the unpacking are in the scale
+    const float s3 = 0.5f * a.scale3, s2 = 0.5f * a.scale2;
+
+    // plane and first row of each pair (those beyond the last repeat it)
+    int2 *at = reinterpret_cast<int2 *>(sm + 2 * IM);
+    for (int r = threadIdx.x; r < RP; r += NT) {
+        const int f = min(f0 + r, F - 1), i3 = f / npr;
+        at[r] = make_int2(i3, 2 * (f - i3 * npr));
+    }
+    __syncthreads();
+
+    // the rows, two by two and 4 points along x1 at a time
+    constexpr int ITS = (RP * R4 + NT - 1) / NT;
+    const int rr0 = threadIdx.x / R4, q0 = threadIdx.x - rr0 * R4;
+    constexpr bool FIXED = NT % R4 == 0;   // a thread keeps its place along the row
+#pragma unroll 2
+    for (int it = 0; it < ITS; it++) {
+        const int q = threadIdx.x + NT * it, rr = FIXED ? rr0 + NT / R4 * it : q / R4;
+        const int x = 4 * (FIXED ? q0 : q - rr * R4);
+        if (RP * R4 % NT && q >= RP * R4) break;
+        const int i3 = at[rr].x, ra = at[rr].y, rb = ra + 1 < g.sx2 ? ra + 1 : ra;
+        float4 fa, fb;
+        if (i3 == a.nin) {   // the surface traction
+            if (XIN == XIN_DIV) {
+                const float *mt = a.m + cz * g.nh + x;
+                fa = ldc4(mt + (size_t)ra * SX1);
+                fb = ldc4(mt + (size_t)rb * SX1);
+            } else {
+                const float *ta = a.tin[c] + (size_t)ra * a.trp + x, *tb = a.tin[c] + (size_t)rb * a.trp + x;
+                fa = make_float4(ta[0], ta[1], ta[2], ta[3]);
+                fb = make_float4(tb[0], tb[1], tb[2], tb[3]);
+            }
+            if (c == 2 && a.tload) {
+                const float4 la = ldc4(a.tload + (size_t)ra * SX1 + x), lb = ldc4(a.tload + (size_t)rb * SX1 + x);
+                fa.x += la.x; fa.y += la.y; fa.z += la.z; fa.w += la.w;
+                fb.x += lb.x; fb.y += lb.y; fb.z += lb.z; fb.w += lb.w;
+            }
+            fa.x *= s2; fa.y *= s2; fa.z *= s2; fa.w *= s2;
+            fb.x *= s2; fb.y *= s2; fb.z *= s2; fb.w *= s2;
+        } else if (XIN == XIN_REAL) {
+            const float *pa = a.in[c] + (size_t)i3 * a.pp + x, *pb = pa + (size_t)rb * a.rp;
+            pa += (size_t)ra * a.rp;
+            fa = make_float4(pa[0] * s3, pa[1] * s3, pa[2] * s3, pa[3] * s3);
+            fb = make_float4(pb[0] * s3, pb[1] * s3, pb[2] * s3, pb[3] * s3);
+        } else {
+            const size_t pl = (size_t)i3 * g.plane;
+            const int rm = ra == 0 ? g.sx2 - 1 : ra - 1, rn = rb + 1 >= g.sx2 ? 0 : rb + 1;
+            const bool top = i3 == 0, bot = i3 == g.sx3h - 1;
+            const float kz = top || bot ? a.k3b : a.k3;
+            const float *mx = a.m + cx * g.nh + pl, *my = a.m + cy * g.nh + pl + x, *mz = a.m + cz * g.nh + pl + x;
+            const float *zp = bot ? mz : mz + g.plane, *zm = top ? mz : mz - g.plane;
+            const size_t oa = (size_t)ra * SX1, ob = (size_t)rb * SX1;
+            const float4 xa = ld4(mx + oa + x), xb = ld4(mx + ob + x);
+            const float4 y0 = ld4(my + (size_t)rm * SX1), y1 = ld4(my + oa), y2 = ld4(my + ob),
+                         y3 = ld4(my + (size_t)rn * SX1);
+            const float4 pa = ld4(zp + oa), na = ld4(zm + oa), pb = ld4(zp + ob), nb = ld4(zm + ob);
+            const int xm = x == 0 ? SX1 - 1 : x - 1, xn = x + 4 == SX1 ? 0 : x + 4;
+            float la, ha, lb, hb;   // x neighbours of the group
+            if (R4 % 32 == 0) {     // a warp's groups are neighbours in one row
+                const int lane = threadIdx.x & 31;
+                la = __shfl_up_sync(0xffffffffu, xa.w, 1);
+                lb = __shfl_up_sync(0xffffffffu, xb.w, 1);
+                ha = __shfl_down_sync(0xffffffffu, xa.x, 1);
+                hb = __shfl_down_sync(0xffffffffu, xb.x, 1);
+                if (lane == 0) { la = __ldg(mx + oa + xm); lb = __ldg(mx + ob + xm); }
+                if (lane == 31) { ha = __ldg(mx + oa + xn); hb = __ldg(mx + ob + xn); }
+            } else {
+                la = __ldg(mx + oa + xm); lb = __ldg(mx + ob + xm);
+                ha = __ldg(mx + oa + xn); hb = __ldg(mx + ob + xn);
+            }
+            const float sk = -s3;
+            // for odd sx2 the last row is alone: its partner repeats it
+            const float4 ya = rb == ra ? y3 : y2;
+            fa.x = ((xa.y - la) * a.k1 + (ya.x - y0.x) * a.k2 + (pa.x - na.x) * kz) * sk;
+            fa.y = ((xa.z - xa.x) * a.k1 + (ya.y - y0.y) * a.k2 + (pa.y - na.y) * kz) * sk;
+            fa.z = ((xa.w - xa.y) * a.k1 + (ya.z - y0.z) * a.k2 + (pa.z - na.z) * kz) * sk;
+            fa.w = ((ha - xa.z) * a.k1 + (ya.w - y0.w) * a.k2 + (pa.w - na.w) * kz) * sk;
+            fb.x = ((xb.y - lb) * a.k1 + (y3.x - y1.x) * a.k2 + (pb.x - nb.x) * kz) * sk;
+            fb.y = ((xb.z - xb.x) * a.k1 + (y3.y - y1.y) * a.k2 + (pb.y - nb.y) * kz) * sk;
+            fb.z = ((xb.w - xb.y) * a.k1 + (y3.z - y1.z) * a.k2 + (pb.z - nb.z) * kz) * sk;
+            fb.w = ((hb - xb.z) * a.k1 + (y3.w - y1.w) * a.k2 + (pb.w - nb.w) * kz) * sk;
+        }
+        float2 *T = sm + rr * RS + x / 2;
+        if (RS % 2 == 0) {
+            *reinterpret_cast<float4 *>(T) = make_float4(fa.x, fb.x, fa.z, fb.z);
+            *reinterpret_cast<float4 *>(T + IM) = make_float4(fa.y, fb.y, fa.w, fb.w);
+        } else {
+            T[0] = make_float2(fa.x, fb.x);
+            T[1] = make_float2(fa.z, fb.z);
+            T[IM] = make_float2(fa.y, fb.y);
+            T[IM + 1] = make_float2(fa.w, fb.w);
+        }
+    }
+    __syncthreads();
+    row_fft<N1, N2, -1>(sm + (threadIdx.x / N2) * RS, IM, threadIdx.x % N2, true, a.pt);
+
+    // X[k] and X[M - k] of both rows from Z[k], Z[M - k]: with e = Z[k] +
+    // conj Z[M-k], d = Z[k] - conj Z[M-k], v = exp(-2 pi i k / sx1) d,
+    // X[k] = e - i v and X[M-k] = conj(e) - i conj(v) (halves in the scale)
+    auto emit = [&](int rr, int k, float2 w) {
+        const int i3 = at[rr].x, ra = at[rr].y, p = i3 == a.nin ? g.sx3 : i3;
+        const float2 *T = sm + rr * RS;
+        const int km = k == 0 ? 0 : M - k;
+        const P2 zk = {T[k], T[k + IM]}, zm = {T[km], T[km + IM]};
+        const P2 e = {add2(zk.r, zm.r), sub2(zk.i, zm.i)}, d = {sub2(zk.r, zm.r), add2(zk.i, zm.i)};
+        const P2 v = pmul<false>(d, W2{f2(w.x), f2(w.y)});
+        const P2 x0 = {add2(e.r, v.i), sub2(e.i, v.r)}, x1 = {sub2(e.r, v.i), neg2(add2(e.i, v.r))};
+        float2 *dst = a.S + sidx(g, c, p, ra, 0);
+        dst[k] = make_float2(x0.r.x, x0.i.x);
+        dst[M - k] = make_float2(x1.r.x, x1.i.x);
+        if (ra + 1 < g.sx2) {
+            dst[g.KP + k] = make_float2(x0.r.y, x0.i.y);
+            dst[g.KP + M - k] = make_float2(x1.r.y, x1.i.y);
+        }
+    };
+    const float2 wf = __ldg(a.tw1 + q0);
+    const int nr = min(RP, F - f0);
+#pragma unroll 2
+    for (int it = 0; it < ITS; it++) {
+        const int q = threadIdx.x + NT * it, rr = FIXED ? rr0 + NT / R4 * it : q / R4;
+        if (rr >= nr) break;
+        const int k = FIXED ? q0 : q - rr * R4;
+        emit(rr, k, FIXED ? wf : __ldg(a.tw1 + k));
+    }
+    for (int rr = threadIdx.x; rr < nr; rr += NT) emit(rr, M / 2, make_float2(0.f, -1.f));   // exp(-i pi / 2)
+}
+
+template <int XIN, int N1, int N2, bool BATCH>
+void launch_fwd(const XfArgs &xa, int nm, cudaStream_t st)
+{
+    const int F = (xa.nin + 1) * ((xa.g.sx2 + 1) / 2), RP = xpairs(N2);
+    auto k = k_xfwd_p<XIN, N1, N2, BATCH>;
+    set_smem(k, xsmem(N1, N2));
+    launch_pdl(k, dim3(3 * ((F + RP - 1) / RP), nm), RP * N2, xsmem(N1, N2), st, xa);
+}
+
+template <int N1, int N2>
+void launch_fwd(const XfArgs &xa, bool div, cudaStream_t st)
+{
+    if (div) launch_fwd<XIN_DIV, N1, N2, false>(xa, 1, st);
+    else launch_fwd<XIN_REAL, N1, N2, false>(xa, 1, st);
+}
+
+}  // namespace
+
+bool xpass_batch_length(int M) { return M == 32 || M == 64 || M == 96 || M == 128 || M == 256; }
+
+// M = sx1/2: the even products of 2 and 3 from 12 to 256; other lengths, and
+// grids of the 7-point differentiators, take k_xfwd.
+bool xfwd_reg(const XfArgs &xa, bool div, cudaStream_t st, cudaError_t *e, int nm)
+{
+    if (div && (xa.fx.n || xa.fy.n)) return false;
+    if (nm > 1) {
+        if (!div) return false;
+        switch (xa.g.M) {
+        case 32: launch_fwd<XIN_DIV, 8, 4, true>(xa, nm, st); break;
+        case 64: launch_fwd<XIN_DIV, 8, 8, true>(xa, nm, st); break;
+        case 96: launch_fwd<XIN_DIV, 12, 8, true>(xa, nm, st); break;
+        case 128: launch_fwd<XIN_DIV, 16, 8, true>(xa, nm, st); break;
+        case 256: launch_fwd<XIN_DIV, 16, 16, true>(xa, nm, st); break;
+        default: return false;
+        }
+        *e = cudaGetLastError();
+        return true;
+    }
+    switch (xa.g.M) {
+    case 12: launch_fwd<4, 3>(xa, div, st); break;
+    case 16: launch_fwd<4, 4>(xa, div, st); break;
+    case 18: launch_fwd<6, 3>(xa, div, st); break;
+    case 24: launch_fwd<6, 4>(xa, div, st); break;
+    case 32: launch_fwd<8, 4>(xa, div, st); break;
+    case 36: launch_fwd<6, 6>(xa, div, st); break;
+    case 48: launch_fwd<12, 4>(xa, div, st); break;
+    case 54: launch_fwd<9, 6>(xa, div, st); break;
+    case 64: launch_fwd<8, 8>(xa, div, st); break;
+    case 72: launch_fwd<12, 6>(xa, div, st); break;
+    case 96: launch_fwd<12, 8>(xa, div, st); break;
+    case 108: launch_fwd<18, 6>(xa, div, st); break;
+    case 128: launch_fwd<16, 8>(xa, div, st); break;
+    case 144: launch_fwd<12, 12>(xa, div, st); break;
+    case 162: launch_fwd<18, 9>(xa, div, st); break;
+    case 192: launch_fwd<24, 8>(xa, div, st); break;
+    case 216: launch_fwd<24, 9>(xa, div, st); break;
+    case 256: launch_fwd<16, 16>(xa, div, st); break;
+    default: return false;
+    }
+    *e = cudaGetLastError();
+    return true;
+}
+
+}  // namespace relax

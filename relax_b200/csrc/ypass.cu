@@ -38,10 +38,12 @@ __global__ void __launch_bounds__(CW *N2, yblocks(N1, N2)) k_ypass_p(const __gri
     const Grid &g = a.g;
     const int c = threadIdx.x % CW, t = threadIdx.x / CW;
     const int KP2 = g.KP / 2, np = a.nbody + a.traction;
-    // pairs flattened: f = (cp np + pi) KP2 + kk
+    // pairs flattened: f = (3 pi + cp) KP2 + kk, the planes from the first to
+    // the last (the x1 passes go the other way: what one pass wrote last is
+    // in L2 when the next begins)
     const int f = blockIdx.x * CW + c;
     const bool ok = f < 3 * np * KP2;
-    const int cpi = ok ? f / KP2 : 0, cp = cpi / np, pi = cpi - cp * np;
+    const int cpi = ok ? f / KP2 : 0, pi = cpi / 3, cp = cpi - 3 * pi;
     const int p = (a.traction && pi == a.nbody) ? g.sx3 : pi;
     float4 *S = reinterpret_cast<float4 *>(a.S + sidx(g, cp, p, 0, 0)) + (ok ? f - cpi * KP2 : 0);
     // 8-byte accesses of a half-warp are two runs of CW pairs: the swizzle

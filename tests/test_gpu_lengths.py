@@ -23,6 +23,7 @@ torch = pytest.importorskip("torch")
 
 X3 = (24, 32, 36, 48, 54, 64, 72, 96, 108, 128, 144, 162, 192, 216, 256, 288, 384, 512)
 X2 = (24, 27, 32, 36, 48, 54, 64, 72, 81, 96, 108, 128, 144, 162, 192, 216, 243, 256, 288, 324, 384, 432, 486, 512)
+X1 = (24, 32, 36, 48, 64, 72, 96, 108, 128, 144, 192, 216, 256, 288, 324, 384, 432, 512)
 
 
 def green_error(oracle, sx1, sx2, sx3, gam=8.3e-4):
@@ -65,3 +66,10 @@ def test_x3_lengths(oracle32, sx3):
 @pytest.mark.parametrize("sx2", X2)
 def test_x2_lengths(oracle32, sx2):
     assert green_error(oracle32, 24, sx2, 32) < 1e-5
+
+
+@pytest.mark.parametrize("sx1", X1)
+def test_x1_lengths(oracle32, sx1):
+    assert green_error(oracle32, sx1, 18, 24) < 1e-5
+    errs = step_errors(oracle32, sx1, 27, 24)            # odd sx2: the last row of a plane has no partner
+    assert max(errs.values()) < 1e-5, errs
