@@ -6,7 +6,6 @@
 #pragma once
 
 #include "common.cuh"
-#include "rfft.cuh"
 #include "spectral.cuh"
 
 namespace relax {
@@ -1392,123 +1391,6 @@ __global__ void __launch_bounds__(RELAX_NTHREADS) k_xinv(XiArgs a)
     }
 }
 
-
-// pass 5, register-resident: C2R along x1 for rows of M = N1*N2 complex
-// values, RW rows of one plane and one component per block, N2 threads per
-// row, with the field update out = base + coef * w.  Shared-memory rows are
-// padded (N2+1 per k1 group, row stride = 8 mod 16 float2) so both transpose
-// access patterns are free of bank conflicts.  Register budgets as measured:
-// 3 blocks per SM for M = 128 (33.6 -> 32.5 us on the 256 x 256 x 128 box),
-// the registers asked for at M = 64.
-template <int N1, int N2, int RW, int V, bool BATCH = false>
-__global__ void __launch_bounds__(RW *N2, (N1 * N2 == 128) ? 3 : (N1 * N2 == 64) ? 1 : 0) k_xinv_reg(const __grid_constant__ XiArgs a0)
-{
-    pdl_enter();
-    const XiArgs &a = BATCH ? a0.tab[blockIdx.z / 3] : a0;
-    // RW rows of one plane and component per block, N2 threads per row.
-    // (A) the block's spectrum rows, one contiguous run of RW*KP values
-    //     in S, are staged in shared memory with 16-byte loads;
-    // (B) each row thread unpacks its stride-N2 inputs, transforms in
-    //     registers and leaves the real row in shared memory;
-    // (C) out = base + coef * scale * row with V-wide accesses (V = 4 for
-    //     16-byte aligned rows, else 2).
-    constexpr int M = N1 * N2, Q = N1 / N2, N2P = N2 + 1, KP = M + 2, NT = RW * N2, SX1 = 2 * M;
-    constexpr int RS0 = (N1 * N2P > KP ? N1 * N2P : KP), RS = RS0 + ((8 - RS0 % 16) + 16) % 16;
-    static_assert(N1 % N2 == 0, "N1 must be a multiple of N2");
-    static_assert(RS % 2 == 0 && M % 2 == 0, "float4 staging");
-    static_assert(V == 2 || V == 4, "V");
-    extern __shared__ float2 smx[];
-    const Grid &g = a.g;
-    const int t = threadIdx.x % N2, r = threadIdx.x / N2;
-    const int i2b = blockIdx.x * RW, i3 = blockIdx.y, c = blockIdx.z % 3;
-
-    // (A) rows i2b .. i2b+RW-1 are contiguous: sidx is linear in i2
-    {
-        const float4 *src = reinterpret_cast<const float4 *>(a.S + sidx(g, c, i3, i2b, 0));
-        constexpr int NF = RW * KP / 2, ITS = (NF + NT - 1) / NT;
-#pragma unroll
-        for (int it = 0; it < ITS; it++) {
-            const int f = threadIdx.x + NT * it;
-            if (f < NF) {
-                const float4 v = __ldg(src + f);
-                const int e0 = 2 * f, e1 = 2 * f + 1;
-                smx[(e0 / KP) * RS + e0 % KP] = make_float2(v.x, v.y);
-                smx[(e1 / KP) * RS + e1 % KP] = make_float2(v.z, v.w);
-            }
-        }
-    }
-    __syncthreads();
-    float2 *T = smx + r * RS;
-    float2 x[N1];
-#pragma unroll
-    for (int j1 = 0; j1 < N1; j1++) {
-        const int k = N2 * j1 + t;
-        float2 xk = T[k], xm = T[M - k];
-        if (k == 0) { xk.y = 0.f; xm.y = 0.f; }
-        const float2 e = cscale(cadd(xk, cconj(xm)), 0.5f);
-        const float2 d = cscale(csub(xk, cconj(xm)), 0.5f);
-        const float2 o = cmul(d, cconj(__ldg(&a.tw1[k])));
-        x[j1] = make_float2(e.x - o.y, e.y + o.x);   // E + i O
-    }
-    __syncthreads();
-    RDft<N1, +1>::run(x);
-#pragma unroll
-    for (int k1 = 1; k1 < N1; k1++)
-        if (t) x[k1] = cmul(x[k1], twn<+1>(a.pm.tw, t * k1));
-#pragma unroll
-    for (int k1 = 0; k1 < N1; k1++) T[k1 * N2P + t] = x[k1];
-    __syncthreads();
-    float2 y[Q][N2];
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-        const int k1 = t + N2 * q;
-#pragma unroll
-        for (int jj = 0; jj < N2; jj++) y[q][jj] = T[k1 * N2P + jj];
-        RDft<N2, +1>::run(y[q]);
-    }
-    __syncthreads();
-    // real row in natural order: float2 nn holds x1 = 2 nn, 2 nn + 1
-#pragma unroll
-    for (int q = 0; q < Q; q++)
-#pragma unroll
-        for (int k2 = 0; k2 < N2; k2++) T[(t + N2 * q) + N1 * k2] = y[q][k2];
-    __syncthreads();
-
-    // (C)
-    const float coef = a.st ? (float)(a.cmul * a.st->Dt) : a.cmul;
-    float *out = a.out[c];
-    const float *bs = a.base[c];
-    float *vo = i3 < a.vplanes ? a.vout[c] : nullptr;
-    constexpr int RV = SX1 / V, ITC = RW * RV / NT;
-    static_assert((RW * RV) % NT == 0, "rows split evenly");
-#pragma unroll
-    for (int it = 0; it < ITC; it++) {
-        const int f = threadIdx.x + NT * it, rr = f / RV, x0 = V * (f % RV);
-        const size_t o = (size_t)i3 * a.pp + (size_t)(i2b + rr) * a.rp + x0;
-        const float *row = reinterpret_cast<const float *>(smx + rr * RS) + x0;
-        if (V == 4) {
-            const float4 w4 = *reinterpret_cast<const float4 *>(row);
-            float w[4] = {w4.x * a.scale, w4.y * a.scale, w4.z * a.scale, w4.w * a.scale};
-            if (vo) *reinterpret_cast<float4 *>(vo + o) = make_float4(w[0], w[1], w[2], w[3]);
-            if (bs) {
-                const float4 b = __ldg(reinterpret_cast<const float4 *>(bs + o));
-                w[0] = b.x + coef * w[0]; w[1] = b.y + coef * w[1];
-                w[2] = b.z + coef * w[2]; w[3] = b.w + coef * w[3];
-            }
-            *reinterpret_cast<float4 *>(out + o) = make_float4(w[0], w[1], w[2], w[3]);
-        } else {
-            const float2 w2 = *reinterpret_cast<const float2 *>(row);
-            float w0 = w2.x * a.scale, w1 = w2.y * a.scale;
-            if (vo) *reinterpret_cast<float2 *>(vo + o) = make_float2(w0, w1);
-            if (bs) {
-                const float2 b = *reinterpret_cast<const float2 *>(bs + o);
-                w0 = b.x + coef * w0;
-                w1 = b.y + coef * w1;
-            }
-            *reinterpret_cast<float2 *>(out + o) = make_float2(w0, w1);
-        }
-    }
-}
 
 // postseismic displacement, src/relax.f90:839-850: ur += Dt v over the
 // planes i3 < nur and inter += Dt v in plane i3s (3 components each; v with

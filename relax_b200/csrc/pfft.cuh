@@ -32,6 +32,14 @@ struct P2 {
 struct W2 {
     float2 x, y;
 };
+// one complex element of one line, for the pass that needs the warps more
+// than the instructions (x1 inverse)
+struct P1 {
+    float r, i;
+};
+struct W1 {
+    float x, y;
+};
 
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
@@ -40,19 +48,30 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
-__device__ __forceinline__ P2 padd(P2 a, P2 b) { return {add2(a.r, b.r), add2(a.i, b.i)}; }
-__device__ __forceinline__ P2 psub(P2 a, P2 b) { return {sub2(a.r, b.r), sub2(a.i, b.i)}; }
+__device__ __forceinline__ float neg2(float a) { return -a; }
+__device__ __forceinline__ float add2(float a, float b) { return a + b; }
+__device__ __forceinline__ float sub2(float a, float b) { return a - b; }
+__device__ __forceinline__ float mul2(float a, float b) { return a * b; }
+__device__ __forceinline__ float fma2(float a, float b, float c) { return fmaf(a, b, c); }
+// the constant a in the type of the second argument's parts
+__device__ __forceinline__ float2 like(float a, float2) { return f2(a); }
+__device__ __forceinline__ float like(float a, float) { return a; }
+
+template <class P>
+__device__ __forceinline__ P padd(P a, P b) { return {add2(a.r, b.r), add2(a.i, b.i)}; }
+template <class P>
+__device__ __forceinline__ P psub(P a, P b) { return {sub2(a.r, b.r), sub2(a.i, b.i)}; }
 // a + S i b
-template <int S>
-__device__ __forceinline__ P2 paddi(P2 a, P2 b)
+template <int S, class P>
+__device__ __forceinline__ P paddi(P a, P b)
 {
-    return S > 0 ? P2{sub2(a.r, b.i), add2(a.i, b.r)} : P2{add2(a.r, b.i), sub2(a.i, b.r)};
+    return S > 0 ? P{sub2(a.r, b.i), add2(a.i, b.r)} : P{add2(a.r, b.i), sub2(a.i, b.r)};
 }
 // a w, or a conj(w) for CONJ
-template <bool CONJ>
-__device__ __forceinline__ P2 pmul(P2 a, W2 w)
+template <bool CONJ, class P, class W>
+__device__ __forceinline__ P pmul(P a, W w)
 {
-    const float2 p = mul2(a.r, w.x), q = mul2(a.i, w.x);
+    const auto p = mul2(a.r, w.x), q = mul2(a.i, w.x);
     if (CONJ) return {fma2(a.i, w.y, p), fma2(neg2(a.r), w.y, q)};
     return {fma2(neg2(a.i), w.y, p), fma2(a.r, w.y, q)};
 }
@@ -132,37 +151,41 @@ __constant__ float4 c_p18[18] = {
 };
 
 // exp(-2 pi i m / R)
+__device__ __forceinline__ W2 wlike(float4 v, P2) { return w2(v); }
+__device__ __forceinline__ W1 wlike(float4 v, P1) { return {v.x, v.z}; }
 template <int R>
-__device__ __forceinline__ W2 pconst(int m)
+__device__ __forceinline__ float4 pconst(int m)
 {
     static_assert(32 % R == 0 || 24 % R == 0 || 27 % R == 0 || 18 % R == 0, "no constants for this length");
-    if (32 % R == 0) return w2(c_p32[m * (32 / R) % 32]);
-    if (24 % R == 0) return w2(c_p24[m * (24 / R) % 24]);
-    if (27 % R == 0) return w2(c_p27[m * (27 / R) % 27]);
-    return w2(c_p18[m * (18 / R) % 18]);
+    if (32 % R == 0) return c_p32[m * (32 / R) % 32];
+    if (24 % R == 0) return c_p24[m * (24 / R) % 24];
+    if (27 % R == 0) return c_p27[m * (27 / R) % 27];
+    return c_p18[m * (18 / R) % 18];
 }
 
-// DFT of R pairs in registers, natural order in and out; the inputs from nz
+// DFT of R values (P2 or P1) in registers, natural order in and out; the inputs from nz
 // on are zero (they are not read), nz a constant after unrolling
 template <int R, int S> struct PDft;
 
 template <int S> struct PDft<2, S> {
-    __device__ __forceinline__ static void run(P2 *v, int nz = 2)
+    template <class P>
+    __device__ __forceinline__ static void run(P *v, int nz = 2)
     {
         if (nz <= 1) { v[1] = v[0]; return; }
-        const P2 a = v[0], b = v[1];
+        const P a = v[0], b = v[1];
         v[0] = padd(a, b);
         v[1] = psub(a, b);
     }
 };
 
 template <int S> struct PDft<3, S> {
-    __device__ __forceinline__ static void run(P2 *v, int nz = 3)
+    template <class P>
+    __device__ __forceinline__ static void run(P *v, int nz = 3)
     {
         if (nz <= 1) { v[1] = v[2] = v[0]; return; }
-        const P2 t = nz <= 2 ? v[1] : padd(v[1], v[2]), d = nz <= 2 ? v[1] : psub(v[1], v[2]);
-        const float2 h = f2(-0.5f), s = f2(S * 0.86602540378443864676f), m = f2(-S * 0.86602540378443864676f);
-        const P2 a = {fma2(t.r, h, v[0].r), fma2(t.i, h, v[0].i)};
+        const P t = nz <= 2 ? v[1] : padd(v[1], v[2]), d = nz <= 2 ? v[1] : psub(v[1], v[2]);
+        const auto h = like(-0.5f, v[0].r), s = like(S * 0.86602540378443864676f, v[0].r), m = neg2(s);
+        const P a = {fma2(t.r, h, v[0].r), fma2(t.i, h, v[0].i)};
         v[0] = padd(v[0], t);
         v[1] = {fma2(d.i, m, a.r), fma2(d.r, s, a.i)};
         v[2] = {fma2(d.i, s, a.r), fma2(d.r, m, a.i)};
@@ -170,12 +193,13 @@ template <int S> struct PDft<3, S> {
 };
 
 template <int S> struct PDft<4, S> {
-    __device__ __forceinline__ static void run(P2 *v, int nz = 4)
+    template <class P>
+    __device__ __forceinline__ static void run(P *v, int nz = 4)
     {
         if (nz <= 1) { v[1] = v[2] = v[3] = v[0]; return; }
-        const P2 a = v[0], b = v[1];
-        const P2 t0 = nz <= 2 ? a : padd(a, v[2]), t1 = nz <= 2 ? a : psub(a, v[2]);
-        const P2 t2 = nz <= 3 ? b : padd(b, v[3]), d = nz <= 3 ? b : psub(b, v[3]);
+        const P a = v[0], b = v[1];
+        const P t0 = nz <= 2 ? a : padd(a, v[2]), t1 = nz <= 2 ? a : psub(a, v[2]);
+        const P t2 = nz <= 3 ? b : padd(b, v[3]), d = nz <= 3 ? b : psub(b, v[3]);
         v[0] = padd(t0, t2);
         v[2] = psub(t0, t2);
         v[1] = paddi<S>(t1, d);
@@ -184,10 +208,11 @@ template <int S> struct PDft<4, S> {
 };
 
 template <int S> struct PDft<8, S> {
-    __device__ __forceinline__ static void run(P2 *v, int nz = 8)
+    template <class P>
+    __device__ __forceinline__ static void run(P *v, int nz = 8)
     {
-        const float2 h = f2(0.70710678118654752440f), mh = f2(-0.70710678118654752440f);
-        P2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+        const auto h = like(0.70710678118654752440f, v[0].r), mh = neg2(h);
+        P e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
         if (nz <= 1) {
 #pragma unroll
             for (int k = 1; k < 8; k++) v[k] = v[0];
@@ -195,7 +220,7 @@ template <int S> struct PDft<8, S> {
         }
         PDft<4, S>::run(e, (nz + 1) / 2);
         PDft<4, S>::run(o, nz / 2);
-        const P2 x1 = paddi<S>(o[1], o[1]), x3 = paddi<-S>(o[3], o[3]);   // (1 + S i) o1, (1 - S i) o3
+        const P x1 = paddi<S>(o[1], o[1]), x3 = paddi<-S>(o[3], o[3]);   // (1 + S i) o1, (1 - S i) o3
         v[0] = padd(e[0], o[0]);
         v[4] = psub(e[0], o[0]);
         v[1] = {fma2(x1.r, h, e[1].r), fma2(x1.i, h, e[1].i)};
@@ -210,10 +235,11 @@ template <int S> struct PDft<8, S> {
 // R = A B: n = n1 + A n2, k = k2 + B k1
 template <int A, int B, int S>
 struct PDftAB {
-    __device__ __forceinline__ static void run(P2 *v, int nz)
+    template <class P>
+    __device__ __forceinline__ static void run(P *v, int nz)
     {
         constexpr int R = A * B;
-        P2 a[A][B];
+        P a[A][B];
 #pragma unroll
         for (int n1 = 0; n1 < A; n1++) {
 #pragma unroll
@@ -223,14 +249,14 @@ struct PDftAB {
             for (int k2 = 1; k2 < B; k2++) {
                 if (n1 == 0) continue;
                 if (4 * n1 * k2 == R)
-                    a[n1][k2] = S > 0 ? P2{neg2(a[n1][k2].i), a[n1][k2].r} : P2{a[n1][k2].i, neg2(a[n1][k2].r)};
+                    a[n1][k2] = S > 0 ? P{neg2(a[n1][k2].i), a[n1][k2].r} : P{a[n1][k2].i, neg2(a[n1][k2].r)};
                 else
-                    a[n1][k2] = pmul<(S > 0)>(a[n1][k2], pconst<R>(n1 * k2));
+                    a[n1][k2] = pmul<(S > 0)>(a[n1][k2], wlike(pconst<R>(n1 * k2), P{}));
             }
         }
 #pragma unroll
         for (int k2 = 0; k2 < B; k2++) {
-            P2 t[A];
+            P t[A];
 #pragma unroll
             for (int n1 = 0; n1 < A; n1++) t[n1] = a[n1][k2];
             PDft<A, S>::run(t);
@@ -240,28 +266,36 @@ struct PDftAB {
     }
 };
 template <int S> struct PDft<6, S> {
-    __device__ __forceinline__ static void run(P2 *v, int nz = 6) { PDftAB<2, 3, S>::run(v, nz); }
+    template <class P>
+    __device__ __forceinline__ static void run(P *v, int nz = 6) { PDftAB<2, 3, S>::run(v, nz); }
 };
 template <int S> struct PDft<9, S> {
-    __device__ __forceinline__ static void run(P2 *v, int nz = 9) { PDftAB<3, 3, S>::run(v, nz); }
+    template <class P>
+    __device__ __forceinline__ static void run(P *v, int nz = 9) { PDftAB<3, 3, S>::run(v, nz); }
 };
 template <int S> struct PDft<12, S> {
-    __device__ __forceinline__ static void run(P2 *v, int nz = 12) { PDftAB<3, 4, S>::run(v, nz); }
+    template <class P>
+    __device__ __forceinline__ static void run(P *v, int nz = 12) { PDftAB<3, 4, S>::run(v, nz); }
 };
 template <int S> struct PDft<16, S> {
-    __device__ __forceinline__ static void run(P2 *v, int nz = 16) { PDftAB<4, 4, S>::run(v, nz); }
+    template <class P>
+    __device__ __forceinline__ static void run(P *v, int nz = 16) { PDftAB<4, 4, S>::run(v, nz); }
 };
 template <int S> struct PDft<18, S> {
-    __device__ __forceinline__ static void run(P2 *v, int nz = 18) { PDftAB<3, 6, S>::run(v, nz); }
+    template <class P>
+    __device__ __forceinline__ static void run(P *v, int nz = 18) { PDftAB<3, 6, S>::run(v, nz); }
 };
 template <int S> struct PDft<24, S> {
-    __device__ __forceinline__ static void run(P2 *v, int nz = 24) { PDftAB<3, 8, S>::run(v, nz); }
+    template <class P>
+    __device__ __forceinline__ static void run(P *v, int nz = 24) { PDftAB<3, 8, S>::run(v, nz); }
 };
 template <int S> struct PDft<27, S> {
-    __device__ __forceinline__ static void run(P2 *v, int nz = 27) { PDftAB<3, 9, S>::run(v, nz); }
+    template <class P>
+    __device__ __forceinline__ static void run(P *v, int nz = 27) { PDftAB<3, 9, S>::run(v, nz); }
 };
 template <int S> struct PDft<32, S> {
-    __device__ __forceinline__ static void run(P2 *v, int nz = 32) { PDftAB<4, 8, S>::run(v, nz); }
+    template <class P>
+    __device__ __forceinline__ static void run(P *v, int nz = 32) { PDftAB<4, 8, S>::run(v, nz); }
 };
 
 }  // namespace

@@ -285,53 +285,6 @@ struct Prof {
         if (prof) (prof)->end(st);                          \
     } while (0)
 
-template <int N1, int N2, int V>
-static void launch_xinv_v(const XiArgs &xi, int nout, size_t sm, int nm, cudaStream_t st)
-{
-    constexpr int RW = 32;
-    if (nm > 1) {
-        set_smem(k_xinv_reg<N1, N2, RW, V, true>, sm);
-        launch_pdl(k_xinv_reg<N1, N2, RW, V, true>, dim3(xi.g.sx2 / RW, nout, 3 * nm), RW * N2, sm, st, xi);
-    } else {
-        set_smem(k_xinv_reg<N1, N2, RW, V>, sm);
-        launch_pdl(k_xinv_reg<N1, N2, RW, V>, dim3(xi.g.sx2 / RW, nout, 3), RW * N2, sm, st, xi);
-    }
-}
-
-template <int N1, int N2>
-static cudaError_t launch_xinv_reg(const XiArgs &xi, int nout, int nm, cudaStream_t st)
-{
-    constexpr int RW = 32, N2P = N2 + 1, KP = N1 * N2 + 2;
-    constexpr int RS0 = (N1 * N2P > KP ? N1 * N2P : KP), RS = RS0 + ((8 - RS0 % 16) + 16) % 16;
-    const size_t sm = (size_t)RW * RS * sizeof(float2);
-    // 16-byte output rows: float4 epilogue (the members of a batch share the layout)
-    bool v4 = xi.rp % 4 == 0 && xi.pp % 4 == 0;
-    for (int k = 0; k < 3; k++) {
-        v4 = v4 && ((uintptr_t)xi.out[k] % 16 == 0);
-        if (xi.base[k]) v4 = v4 && ((uintptr_t)xi.base[k] % 16 == 0);
-    }
-    if (v4) launch_xinv_v<N1, N2, 4>(xi, nout, sm, nm, st);
-    else launch_xinv_v<N1, N2, 2>(xi, nout, sm, nm, st);
-    return cudaGetLastError();
-}
-
-static bool xinv_reg(const XiArgs &xi, int nout, cudaStream_t st, cudaError_t *e, int nm = 1)
-{
-    if (xi.g.sx2 % 32) return false;
-    // the epilogue moves at least float2: even pitches, 8-byte aligned rows
-    if (xi.rp % 2 || xi.pp % 2) return false;
-    for (int k = 0; k < 3; k++)
-        if ((uintptr_t)xi.out[k] % 8 || (uintptr_t)xi.base[k] % 8) return false;
-    switch (xi.g.M) {
-    case 32: *e = launch_xinv_reg<8, 4>(xi, nout, nm, st); return true;
-    case 96: *e = launch_xinv_reg<24, 4>(xi, nout, nm, st); return true;
-    case 64: *e = launch_xinv_reg<8, 8>(xi, nout, nm, st); return true;
-    case 128: *e = launch_xinv_reg<16, 8>(xi, nout, nm, st); return true;
-    case 256: *e = launch_xinv_reg<16, 16>(xi, nout, nm, st); return true;
-    default: return false;
-    }
-}
-
 // the lengths the register passes are instantiated for
 static bool reg_shape(const Grid &g)
 {
@@ -504,8 +457,9 @@ struct Spectral {
         za.lambda = lambda; za.mu = mu; za.gam = gam;
         return za;
     }
-    XiArgs xiargs(XiArgs xi) const
+    XiArgs xiargs(XiArgs xi, int nout) const
     {
+        xi.nout = nout;
         xi.g = g; xi.S = S; xi.pm = pm; xi.pt = ptx; xi.tw1 = tw1; xi.rows = rows;
         xi.scale = (float)(2.0 / ((double)g.sx1 * g.dx1 * g.sx2 * g.dx2 * g.sx3 * g.dx3));
         return xi;
@@ -563,11 +517,11 @@ struct Spectral {
             TIMED(prof, ST_YINV, st,
                   (k_ypass<+1><<<dim3((g.K1 + twy - 1) / twy, nout, 3), RELAX_NTHREADS, smy, st>>>(yb)));
         }
-        xi = xiargs(xi);
+        xi = xiargs(xi, nout);
         if (join_before_xinv) CK(cudaStreamWaitEvent(st, join_before_xinv, 0));
         bool xr = false;
         if (use_reg) {
-            TIMED(prof, ST_XINV, st, (xr = xinv_reg(xi, nout, st, &re)));
+            TIMED(prof, ST_XINV, st, (xr = xinv_reg(xi, st, &re)));
             if (re != cudaSuccess) return fail(RELAX_ERR_CUDA, "k_xinv_reg: %s", cudaGetErrorString(re));
         }
         if (!xr) TIMED(prof, ST_XINV, st, (k_xinv<<<dim3(g.sx2 / rows, nout), RELAX_NTHREADS, smx, st>>>(xi)));
@@ -3477,8 +3431,8 @@ static int build_tables(relax_batch *b)
         yf[k] = c->sp.yargs(g.sx3h, 1, 0);
         yi[k] = c->sp.yargs(g.sx3h, 0, 0);
         z[k] = c->sp.zargs(g.sx3h, g.sx3h, c->cfg.lambda, c->cfg.mu, c->cfg.gam, 0);
-        xip[k] = c->sp.xiargs(xi_update(c, c->vp, c->u, 0.5f, true));
-        xic[k] = c->sp.xiargs(xi_update(c, c->u, c->u, 1.0f, true));
+        xip[k] = c->sp.xiargs(xi_update(c, c->vp, c->u, 0.5f, true), g.sx3h);
+        xic[k] = c->sp.xiargs(xi_update(c, c->u, c->u, 1.0f, true), g.sx3h);
         int tot = 0;
         TRY(friction_slots(c, &tot));
         b->nfr[k] = tot;
@@ -3569,7 +3523,7 @@ static int batch_green(relax_batch *b, const XiArgs &xi0)
         return fail(RELAX_ERR_CUDA, "batched z pass: %s", cudaGetErrorString(e));
     if (!ypass_reg(t.yi0, +1, b->st, &e, n) || e != cudaSuccess)
         return fail(RELAX_ERR_CUDA, "batched y pass: %s", cudaGetErrorString(e));
-    if (!xinv_reg(xi0, g.sx3h, b->st, &e, n) || e != cudaSuccess)
+    if (!xinv_reg(xi0, b->st, &e, n) || e != cudaSuccess)
         return fail(RELAX_ERR_CUDA, "batched x inverse: %s", cudaGetErrorString(e));
     b->launches += 5;
     return RELAX_OK;

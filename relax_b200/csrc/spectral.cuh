@@ -86,9 +86,10 @@ struct XiArgs {
     size_t rp, pp;           // pitches of out/base
     const StepState *st;     // coef = cmul * Dt (or cmul when st is null)
     float cmul, scale;
-    const struct XiArgs *tab;   // batched launch: one entry per member (blockIdx.z / 3)
+    const struct XiArgs *tab;   // batched launch: one entry per member (blockIdx.y)
     float *vout[3];          // optional copy of the transformed field (the
     int vplanes;             // velocity v) for planes i3 < vplanes, pitches rp/pp
+    int nout;                // planes [0, nout) are written
 };
 
 // The register-resident passes: false when the grid's length has no
@@ -97,6 +98,7 @@ struct XiArgs {
 bool xfwd_reg(const XfArgs &xa, bool div, cudaStream_t st, cudaError_t *e, int nm = 1);
 bool ypass_reg(const YArgs &ya, int sign, cudaStream_t st, cudaError_t *e, int nm = 1);
 bool zspec_reg(const ZArgs &za, cudaStream_t st, cudaError_t *e, int nm = 1);
+bool xinv_reg(const XiArgs &xi, cudaStream_t st, cudaError_t *e, int nm = 1);
 // whether the x3 pass is instantiated for a length
 bool zspec_length(int sx3);
 // The table that zspec_reg reads for planes [0, planes): plane stride and

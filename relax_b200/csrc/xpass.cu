@@ -8,8 +8,6 @@
 // side of it; real and imaginary parts (of two rows: 8 bytes) are in separate
 // arrays.  Pairs of rows are numbered through all planes, so that no block
 // is left partly empty at a plane's end.
-#include <cuda_bf16.h>
-
 #include "launch.cuh"
 #include "pfft.cuh"
 #include "spectral.cuh"
@@ -41,49 +39,41 @@ constexpr int xblocks(int N1, int N2, int extra)
 }
 
 // complex transform of the block's row pairs, from T (natural order) to T
-// (natural order); every thread has one pair's t, those beyond the last pair none
+// (natural order), N2 threads a pair
 template <int N1, int N2, int SIGN>
-__device__ __forceinline__ void row_fft(float2 *T, int IM, int t, bool on, const float4 *pt)
+__device__ __forceinline__ void row_fft(float2 *T, int IM, int t, const float4 *pt)
 {
     constexpr int Q = (N1 + N2 - 1) / N2, NP = N2 | 1;
     P2 z[N1];
-    if (on) {
 #pragma unroll
-        for (int j1 = 0; j1 < N1; j1++) z[j1] = {T[N2 * j1 + t], T[N2 * j1 + t + IM]};
-    }
+    for (int j1 = 0; j1 < N1; j1++) z[j1] = {T[N2 * j1 + t], T[N2 * j1 + t + IM]};
     __syncthreads();
-    if (on) {
-        PDft<N1, SIGN>::run(z);
+    PDft<N1, SIGN>::run(z);
 #pragma unroll
-        for (int k1 = 0; k1 < N1; k1++) {
-            const P2 v = k1 ? pmul<(SIGN > 0)>(z[k1], w2(__ldg(pt + t * k1))) : z[k1];
-            T[k1 * NP + t] = v.r;
-            T[k1 * NP + t + IM] = v.i;
-        }
+    for (int k1 = 0; k1 < N1; k1++) {
+        const P2 v = k1 ? pmul<(SIGN > 0)>(z[k1], w2(__ldg(pt + t * k1))) : z[k1];
+        T[k1 * NP + t] = v.r;
+        T[k1 * NP + t + IM] = v.i;
     }
     __syncthreads();
     P2 y[Q][N2];
-    if (on) {
 #pragma unroll
-        for (int q = 0; q < Q; q++) {
-            const int k1 = t + N2 * q;
-            if (N1 % N2 && k1 >= N1) break;
+    for (int q = 0; q < Q; q++) {
+        const int k1 = t + N2 * q;
+        if (N1 % N2 && k1 >= N1) break;
 #pragma unroll
-            for (int jj = 0; jj < N2; jj++) y[q][jj] = {T[k1 * NP + jj], T[k1 * NP + jj + IM]};
-            PDft<N2, SIGN>::run(y[q]);
-        }
+        for (int jj = 0; jj < N2; jj++) y[q][jj] = {T[k1 * NP + jj], T[k1 * NP + jj + IM]};
+        PDft<N2, SIGN>::run(y[q]);
     }
     __syncthreads();
-    if (on) {
 #pragma unroll
-        for (int q = 0; q < Q; q++) {
-            const int k1 = t + N2 * q;
-            if (N1 % N2 && k1 >= N1) break;
+    for (int q = 0; q < Q; q++) {
+        const int k1 = t + N2 * q;
+        if (N1 % N2 && k1 >= N1) break;
 #pragma unroll
-            for (int k2 = 0; k2 < N2; k2++) {
-                T[k1 + N1 * k2] = y[q][k2].r;
-                T[k1 + N1 * k2 + IM] = y[q][k2].i;
-            }
+        for (int k2 = 0; k2 < N2; k2++) {
+            T[k1 + N1 * k2] = y[q][k2].r;
+            T[k1 + N1 * k2 + IM] = y[q][k2].i;
         }
     }
     __syncthreads();
@@ -207,7 +197,7 @@ __global__ void __launch_bounds__(xpairs(N2) *N2, xblocks(N1, N2, 60)) k_xfwd_p(
         }
     }
     __syncthreads();
-    row_fft<N1, N2, -1>(sm + (threadIdx.x / N2) * RS, IM, threadIdx.x % N2, true, a.pt);
+    row_fft<N1, N2, -1>(sm + (threadIdx.x / N2) * RS, IM, threadIdx.x % N2, a.pt);
 
     // X[k] and X[M - k] of both rows from Z[k], Z[M - k]: with e = Z[k] +
     // conj Z[M-k], d = Z[k] - conj Z[M-k], v = exp(-2 pi i k / sx1) d,
@@ -256,6 +246,177 @@ void launch_fwd(const XfArgs &xa, bool div, cudaStream_t st)
     else launch_fwd<XIN_REAL, N1, N2, false>(xa, 1, st);
 }
 
+// Pass 5: C2R along x1 with the field update out = base + coef w (fieldadd,
+// src/elastic3d.f90:3774-3812), or out = w.  V = 4: 16-byte rows, else 2.
+//
+// The pass waits on its loads (the spectrum, then base), so it needs the
+// warps more than it needs fewer instructions: one row per N2 threads, rows
+// numbered through the planes of a component (their spectrum is one run of
+// memory).  Two rows per thread as in pass 1 measured 40.7 instead of 37.4 us
+// on the 256 x 256 x 128 box, 281 instead of 219 us on 512 x 512 x 256.  The
+// planes go from the last to the first, so that the stress pass after it
+// finds the first ones in L2.  109 -> 39 us on 288 x 216 x 144 against the
+// general kernel, 246 -> 219 us on 512 x 512 x 256 against whole rows of one
+// plane and component per block in the planes' order.
+__host__ __device__ constexpr int irows(int N2) { return 128 / N2; }
+__host__ __device__ constexpr int ipitch(int N1, int N2)
+{
+    const int r = N1 * (N2 | 1), n = r > N1 * N2 + 2 ? r : N1 * N2 + 2;
+    const int p = n + ((N2 - n) % 16 + 16) % 16;
+    return p + p % 2;   // rows start on 16 bytes
+}
+__host__ __device__ constexpr size_t ismem(int N1, int N2) { return (size_t)irows(N2) * (ipitch(N1, N2) * 8 + 16); }
+constexpr int iblocks(int N1, int N2)
+{
+    const int sm = (int)(233472 / (ismem(N1, N2) + 1024));
+    const int rg = 65536 / ((2 * (N1 > N2 ? N1 : N2) + 48) * ((irows(N2) * N2 + 31) / 32 * 32));
+    const int m = sm < rg ? sm : rg;
+    return m < 1 ? 1 : m > 16 ? 16 : m;
+}
+
+template <int N1, int N2, int V, bool BATCH>
+__global__ void __launch_bounds__(irows(N2) *N2, iblocks(N1, N2)) k_xinv_r(const __grid_constant__ XiArgs a0)
+{
+    pdl_enter();
+    const XiArgs &a = BATCH ? a0.tab[blockIdx.y] : a0;
+    constexpr int M = N1 * N2, Q = (N1 + N2 - 1) / N2, NP = N2 | 1, KP = M + 2, SX1 = 2 * M, R4 = SX1 / 4;
+    constexpr int RW = irows(N2), NT = RW * N2, RS = ipitch(N1, N2);
+    extern __shared__ __align__(16) float2 sm[];
+    const Grid &g = a.g;
+    const int t = threadIdx.x % N2, r = threadIdx.x / N2;
+    const int c = blockIdx.x % 3, f0 = (gridDim.x / 3 - 1 - blockIdx.x / 3) * RW;
+    const int F = a.nout * g.sx2, nr = min(RW, F - f0);
+    // where the rows go, and their planes
+    size_t *at = reinterpret_cast<size_t *>(sm + RW * RS);
+    int *pl = reinterpret_cast<int *>(at + RW);
+    for (int s = threadIdx.x; s < RW; s += NT) {
+        const int f = min(f0 + s, F - 1), i3 = f / g.sx2;
+        at[s] = (size_t)i3 * a.pp + (size_t)(f - i3 * g.sx2) * a.rp;
+        pl[s] = i3;
+    }
+    // (A) the spectrum rows, 16 bytes at a time
+    {
+        const float4 *src = reinterpret_cast<const float4 *>(a.S + sidx(g, c, 0, 0, 0) + (size_t)f0 * KP);
+        constexpr int NF = RW * KP / 2, ITS = (NF + NT - 1) / NT;
+        const int n = nr * KP / 2;
+#pragma unroll
+        for (int it = 0; it < ITS; it++) {
+            const int f = threadIdx.x + NT * it;
+            if (f < n) *reinterpret_cast<float4 *>(sm + 2 * f / KP * RS + 2 * f % KP) = __ldg(src + f);
+        }
+    }
+    __syncthreads();
+    // (B) Z[k] = (e + i o) / 2 with e = X[k] + conj X[M-k], o = exp(2 pi i k /
+    // sx1) (X[k] - conj X[M-k]) (the half is in the scale; the imaginary parts
+    // of X[0] and X[M] are ignored), transformed and left in natural order
+    float2 *T = sm + r * RS;
+    P1 z[N1];
+#pragma unroll
+    for (int j1 = 0; j1 < N1; j1++) {
+        const int k = N2 * j1 + t;
+        float2 xk = T[k], xm = T[M - k];
+        if (k == 0) xk.y = xm.y = 0.f;
+        const P1 d = {xk.x - xm.x, xk.y + xm.y};
+        const float2 w = __ldg(a.tw1 + k);
+        const P1 o = pmul<true>(d, W1{w.x, w.y});
+        z[j1] = {xk.x + xm.x - o.i, xk.y - xm.y + o.r};
+    }
+    __syncthreads();
+    PDft<N1, +1>::run(z);
+#pragma unroll
+    for (int k1 = 0; k1 < N1; k1++) {
+        if (k1) {
+            const float2 w = __ldg(a.pm.tw + t * k1);
+            z[k1] = pmul<true>(z[k1], W1{w.x, w.y});
+        }
+        T[k1 * NP + t] = make_float2(z[k1].r, z[k1].i);
+    }
+    __syncthreads();
+    P1 y[Q][N2];
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+        const int k1 = t + N2 * q;
+        if (N1 % N2 && k1 >= N1) break;
+#pragma unroll
+        for (int jj = 0; jj < N2; jj++) {
+            const float2 v = T[k1 * NP + jj];
+            y[q][jj] = {v.x, v.y};
+        }
+        PDft<N2, +1>::run(y[q]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+        const int k1 = t + N2 * q;
+        if (N1 % N2 && k1 >= N1) break;
+#pragma unroll
+        for (int k2 = 0; k2 < N2; k2++) T[k1 + N1 * k2] = make_float2(y[q][k2].r, y[q][k2].i);
+    }
+    __syncthreads();
+
+    // (C) the update, CH groups of 4 points at a time: what it reads first
+    // (out may be base, which would keep later loads behind earlier stores)
+    const float coef = a.st ? (float)(a.cmul * a.st->Dt) : a.cmul, scale = 0.5f * a.scale;
+    float *out = a.out[c];
+    const float *bs = a.base[c];
+    constexpr int ITS = (RW * R4 + NT - 1) / NT, CH = ITS < 8 ? ITS : 8;
+    const int rr0 = threadIdx.x / R4, q0 = threadIdx.x - rr0 * R4;
+    constexpr bool FIXED = NT % R4 == 0;   // a thread keeps its place along the row
+#pragma unroll
+    for (int i0 = 0; i0 < ITS; i0 += CH) {
+        float4 b[CH];
+#pragma unroll
+        for (int i = 0; i < CH; i++) {
+            const int q = threadIdx.x + NT * (i0 + i), rr = FIXED ? rr0 + NT / R4 * (i0 + i) : q / R4;
+            if (rr >= nr || !bs) continue;
+            const size_t o = at[rr] + 4 * (FIXED ? q0 : q - rr * R4);
+            if (V == 4) {
+                b[i] = ldc4(bs + o);
+            } else {
+                const float2 u = *reinterpret_cast<const float2 *>(bs + o), v = *reinterpret_cast<const float2 *>(bs + o + 2);
+                b[i] = make_float4(u.x, u.y, v.x, v.y);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < CH; i++) {
+            const int q = threadIdx.x + NT * (i0 + i), rr = FIXED ? rr0 + NT / R4 * (i0 + i) : q / R4;
+            if (rr >= nr) continue;
+            const int x = 4 * (FIXED ? q0 : q - rr * R4);
+            const size_t o = at[rr] + x;
+            const float4 w4 = *reinterpret_cast<const float4 *>(sm + rr * RS + x / 2);
+            float w[4] = {w4.x * scale, w4.y * scale, w4.z * scale, w4.w * scale};
+            auto store = [&](float *dst) {
+                if (V == 4) {
+                    st4(dst, make_float4(w[0], w[1], w[2], w[3]));
+                } else {
+                    *reinterpret_cast<float2 *>(dst) = make_float2(w[0], w[1]);
+                    *reinterpret_cast<float2 *>(dst + 2) = make_float2(w[2], w[3]);
+                }
+            };
+            if (a.vout[c] && pl[rr] < a.vplanes) store(a.vout[c] + o);
+            if (bs) {
+                const float bb[4] = {b[i].x, b[i].y, b[i].z, b[i].w};
+#pragma unroll
+                for (int j = 0; j < 4; j++) w[j] = bb[j] + coef * w[j];
+            }
+            store(out + o);
+        }
+    }
+}
+
+template <int N1, int N2, bool BATCH>
+void launch_inv(const XiArgs &xi, int nm, cudaStream_t st)
+{
+    // 16-byte rows (the members of a batch share the layout)
+    bool v4 = xi.rp % 4 == 0 && xi.pp % 4 == 0;
+    for (int k = 0; k < 3; k++)
+        v4 = v4 && (uintptr_t)xi.out[k] % 16 == 0 && (uintptr_t)xi.base[k] % 16 == 0 && (uintptr_t)xi.vout[k] % 16 == 0;
+    const int F = xi.nout * xi.g.sx2, RW = irows(N2);
+    auto k = v4 ? k_xinv_r<N1, N2, 4, BATCH> : k_xinv_r<N1, N2, 2, BATCH>;
+    set_smem(k, ismem(N1, N2));
+    launch_pdl(k, dim3(3 * ((F + RW - 1) / RW), nm), RW * N2, ismem(N1, N2), st, xi);
+}
+
 }  // namespace
 
 bool xpass_batch_length(int M) { return M == 32 || M == 64 || M == 96 || M == 128 || M == 256; }
@@ -297,6 +458,49 @@ bool xfwd_reg(const XfArgs &xa, bool div, cudaStream_t st, cudaError_t *e, int n
     case 192: launch_fwd<24, 8>(xa, div, st); break;
     case 216: launch_fwd<24, 9>(xa, div, st); break;
     case 256: launch_fwd<16, 16>(xa, div, st); break;
+    default: return false;
+    }
+    *e = cudaGetLastError();
+    return true;
+}
+
+bool xinv_reg(const XiArgs &xi, cudaStream_t st, cudaError_t *e, int nm)
+{
+    // the epilogue moves at least float2: even pitches, 8-byte aligned rows
+    if (xi.rp % 2 || xi.pp % 2) return false;
+    for (int k = 0; k < 3; k++)
+        if ((uintptr_t)xi.out[k] % 8 || (uintptr_t)xi.base[k] % 8) return false;
+    if (nm > 1) {
+        switch (xi.g.M) {
+        case 32: launch_inv<8, 4, true>(xi, nm, st); break;
+        case 64: launch_inv<8, 8, true>(xi, nm, st); break;
+        case 96: launch_inv<12, 8, true>(xi, nm, st); break;
+        case 128: launch_inv<16, 8, true>(xi, nm, st); break;
+        case 256: launch_inv<16, 16, true>(xi, nm, st); break;
+        default: return false;
+        }
+        *e = cudaGetLastError();
+        return true;
+    }
+    switch (xi.g.M) {
+    case 12: launch_inv<4, 3, false>(xi, nm, st); break;
+    case 16: launch_inv<4, 4, false>(xi, nm, st); break;
+    case 18: launch_inv<6, 3, false>(xi, nm, st); break;
+    case 24: launch_inv<6, 4, false>(xi, nm, st); break;
+    case 32: launch_inv<8, 4, false>(xi, nm, st); break;
+    case 36: launch_inv<6, 6, false>(xi, nm, st); break;
+    case 48: launch_inv<12, 4, false>(xi, nm, st); break;
+    case 54: launch_inv<9, 6, false>(xi, nm, st); break;
+    case 64: launch_inv<8, 8, false>(xi, nm, st); break;
+    case 72: launch_inv<12, 6, false>(xi, nm, st); break;
+    case 96: launch_inv<12, 8, false>(xi, nm, st); break;
+    case 108: launch_inv<18, 6, false>(xi, nm, st); break;
+    case 128: launch_inv<16, 8, false>(xi, nm, st); break;
+    case 144: launch_inv<12, 12, false>(xi, nm, st); break;
+    case 162: launch_inv<18, 9, false>(xi, nm, st); break;
+    case 192: launch_inv<24, 8, false>(xi, nm, st); break;
+    case 216: launch_inv<24, 9, false>(xi, nm, st); break;
+    case 256: launch_inv<16, 16, false>(xi, nm, st); break;
     default: return false;
     }
     *e = cudaGetLastError();
