@@ -5,6 +5,7 @@
 // {s11,s12,s13,s22,s23,s33} of nh floats, a vector field 3 planes.
 #pragma once
 
+#include "async.cuh"
 #include "common.cuh"
 #include "spectral.cuh"
 
@@ -183,6 +184,7 @@ struct StressArgs {
     unsigned *ticket;        // INIT/END: blocks done (zero between launches), or null
     StepState *fin;          // with ticket: receives tmin, power, cei
     double dv;               // cell volume dx1 dx2 dx3 (amplitude scale)
+    int *err;                // device error flags (k_stress_pipe)
     const struct StressArgs *tab;   // batched launch: one entry per member (blockIdx.y)
     // transient (Burgers) rheology, TRANS instantiations only
     const TransLayer *trans[2];      // linear / nonlinear transient structures or null
@@ -199,336 +201,346 @@ struct StressArgs {
 // epsilonik += Dt epsilonikdot (:789).
 // FIR: the x1 and x2 derivatives of w come from a.wx, a.wy (k_fir_xy, grids
 // where x1 or x2 takes the 7-point filter) instead of the central differences.
-template <int MODE, bool BATCH = false, bool TRANS = false, bool FIR = false>
-__global__ void __launch_bounds__(RELAX_NTHREADS, TRANS ? 2 : 3) k_stress(const __grid_constant__ StressArgs a0)
+// tau and m of a group of 4 points, read where they are used
+struct FromGlobal {
+    __device__ __forceinline__ float4 tau(const StressArgs &a, int c, size_t idx) const { return ldc4(a.tau + c * a.g.nh + idx); }
+    __device__ __forceinline__ float4 m(const StressArgs &a, int c, size_t idx) const { return ldc4(a.m + c * a.g.nh + idx); }
+};
+// or in registers already
+struct FromRegs {
+    float4 t[6], v[6];
+    __device__ __forceinline__ float4 tau(const StressArgs &, int c, size_t) const { return t[c]; }
+    __device__ __forceinline__ float4 m(const StressArgs &, int c, size_t) const { return v[c]; }
+};
+
+// the group q (4 points along x1) of one stress pass
+template <int MODE, bool TRANS, bool FIR, class SRC>
+__device__ __forceinline__ void stress_group(const StressArgs &a, size_t q, const SRC &src, float (&tmin)[4],
+                                             double &amp_m, double &amp_t)
 {
-    pdl_enter();
-    const StressArgs &a = BATCH ? a0.tab[blockIdx.y] : a0;
-    __shared__ float shf[32];
-    __shared__ double shd[32];
-    if (MODE == MODE_END && a.st->fire) return;   // the event branch of the step runs instead
     const Grid &g = a.g;
-    const int q4 = g.sx1 >> 2;
-    const size_t nq = g.nh >> 2;
-    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = q < nq;
-    constexpr int NTM = TRANS ? 4 : 2;        // Maxwell-time minima: viscous 2 (+ transient 2)
-    float tmin[4] = {3.0e38f, 3.0e38f, 3.0e38f, 3.0e38f};
-    double amp_m = 0.0, amp_t = 0.0;
+    // (read ahead of the rest: a load at the store waited for memory alone)
+    const bool keep = MODE == MODE_OP || (MODE != MODE_EIGEN && a.store_sig && (!a.sig_mask || __ldg(a.sig_mask + q)));
+    // point indexes by 32-bit division (nh / 4 < 2^32) and the periodic
+    // neighbours by selects: no 64-bit division on the device
+    const unsigned qq = (unsigned)q, q4u = (unsigned)(g.sx1 >> 2), sx2u = (unsigned)g.sx2;
+    const unsigned r = qq / q4u, r3 = r / sx2u;
+    const int i1 = (int)(qq - r * q4u) * 4;
+    const int i2 = (int)(r - r3 * sx2u), i3 = (int)r3;
+    const size_t nh = g.nh;
+    const size_t row = ((size_t)i3 * g.sx2 + i2) * g.sx1;
+    const size_t idx = row + i1;
+    const int i1m = i1 == 0 ? g.sx1 - 1 : i1 - 1, i1p = i1 + 4 == g.sx1 ? 0 : i1 + 4;
+    const int i2m = i2 == 0 ? g.sx2 - 1 : i2 - 1, i2p = i2 + 1 == g.sx2 ? 0 : i2 + 1;
+    const size_t rym = ((size_t)i3 * g.sx2 + i2m) * g.sx1 + i1;
+    const size_t ryp = ((size_t)i3 * g.sx2 + i2p) * g.sx1 + i1;
+    size_t rzm, rzp;
+    float kz;
+    if (i3 == 0) { rzm = idx; rzp = idx + g.plane; kz = a.k3b; }
+    else if (i3 == g.sx3h - 1) { rzm = idx - g.plane; rzp = idx; kz = a.k3b; }
+    else { rzm = idx - g.plane; rzp = idx + g.plane; kz = a.k3; }
 
-    if (live) {
-        // point indexes by 32-bit division (nh / 4 < 2^32) and the periodic
-        // neighbours by selects: no 64-bit division on the device
-        const unsigned qq = (unsigned)q, q4u = (unsigned)q4, sx2u = (unsigned)g.sx2;
-        const unsigned r = qq / q4u, r3 = r / sx2u;
-        const int i1 = (int)(qq - r * q4u) * 4;
-        const int i2 = (int)(r - r3 * sx2u), i3 = (int)r3;
-        const size_t nh = g.nh;
-        const size_t row = ((size_t)i3 * g.sx2 + i2) * g.sx1;
-        const size_t idx = row + i1;
-        const int i1m = i1 == 0 ? g.sx1 - 1 : i1 - 1, i1p = i1 + 4 == g.sx1 ? 0 : i1 + 4;
-        const int i2m = i2 == 0 ? g.sx2 - 1 : i2 - 1, i2p = i2 + 1 == g.sx2 ? 0 : i2 + 1;
-        const size_t rym = ((size_t)i3 * g.sx2 + i2m) * g.sx1 + i1;
-        const size_t ryp = ((size_t)i3 * g.sx2 + i2p) * g.sx1 + i1;
-        size_t rzm, rzp;
-        float kz;
-        if (i3 == 0) { rzm = idx; rzp = idx + g.plane; kz = a.k3b; }
-        else if (i3 == g.sx3h - 1) { rzm = idx - g.plane; rzp = idx; kz = a.k3b; }
-        else { rzm = idx - g.plane; rzp = idx + g.plane; kz = a.k3; }
-
-        // END: tau += Dt m first, with every load of tau and m issued before
-        // the stores of tau (which could alias them), so that the kernel waits
-        // for memory once here and once for the strain source below
-        float tn[6][4];
-        if (MODE == MODE_END) {
-            const float dt = (float)a.st->Dt;
-            float4 tv[6], mv[6];
+    // END: tau += Dt m first, with every load of tau and m issued before
+    // the stores of tau (which could alias them), so that the kernel waits
+    // for memory once here and once for the strain source below
+    float tn[6][4];
+    if (MODE == MODE_END) {
+        const float dt = (float)a.st->Dt;
+        float4 tv[6], mv[6];
 #pragma unroll
-            for (int c = 0; c < 6; c++) {
-                tv[c] = ldc4(a.tau + c * nh + idx);
-                mv[c] = ldc4(a.m + c * nh + idx);
-            }
-            constexpr float wn[6] = {1.f, 2.f, 2.f, 1.f, 2.f, 1.f};
-            float qm[4], qt[4];
+        for (int c = 0; c < 6; c++) {
+            tv[c] = src.tau(a, c, idx);
+            mv[c] = src.m(a, c, idx);
+        }
+        constexpr float wn[6] = {1.f, 2.f, 2.f, 1.f, 2.f, 1.f};
+        float qm[4], qt[4];
 #pragma unroll
-            for (int c = 0; c < 6; c++) {
-                const float m4[4] = {mv[c].x, mv[c].y, mv[c].z, mv[c].w};
-                const float t4[4] = {tv[c].x, tv[c].y, tv[c].z, tv[c].w};
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    tn[c][j] = t4[j] + dt * m4[j];
-                    qm[j] = c == 0 ? m4[j] * m4[j] : qm[j] + wn[c] * m4[j] * m4[j];
-                    qt[j] = c == 0 ? tn[c][j] * tn[c][j] : qt[j] + wn[c] * tn[c][j] * tn[c][j];
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < 6; c++)
-                st4(a.tau + c * nh + idx, make_float4(tn[c][0], tn[c][1], tn[c][2], tn[c][3]));
+        for (int c = 0; c < 6; c++) {
+            const float m4[4] = {mv[c].x, mv[c].y, mv[c].z, mv[c].w};
+            const float t4[4] = {tv[c].x, tv[c].y, tv[c].z, tv[c].w};
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                amp_m += (double)sqrtf(qm[j] * 0.5f);
-                amp_t += (double)sqrtf(qt[j] * 0.5f);
+                tn[c][j] = t4[j] + dt * m4[j];
+                qm[j] = c == 0 ? m4[j] * m4[j] : qm[j] + wn[c] * m4[j] * m4[j];
+                qt[j] = c == 0 ? tn[c][j] * tn[c][j] : qt[j] + wn[c] * tn[c][j] * tn[c][j];
             }
         }
-
-        // Hooke's law (src/elastic3d.f90:129-142) on the strain of w at 4
-        // points; h = C:E is added to the base stress below
-        float h[6][4];
-        if (MODE != MODE_EIGEN) {
-            float dxw[3][4], dyw[3][4], dzw[3][4];
 #pragma unroll
-            for (int c = 0; c < 3; c++) {
-                const float *wc = a.w + c * nh;
-                if (FIR) {
-                    const float4 d = ld4(a.wx + c * nh + idx);
-                    dxw[c][0] = d.x; dxw[c][1] = d.y; dxw[c][2] = d.z; dxw[c][3] = d.w;
-                } else {
-                    const float4 cv = ld4(wc + idx);
-                    const float lft = __ldg(wc + row + i1m), rgt = __ldg(wc + row + i1p);
-                    dxw[c][0] = (cv.y - lft) * a.k1;
-                    dxw[c][1] = (cv.z - cv.x) * a.k1;
-                    dxw[c][2] = (cv.w - cv.y) * a.k1;
-                    dxw[c][3] = (rgt - cv.z) * a.k1;
-                }
-                if (FIR) {
-                    const float4 d = ld4(a.wy + c * nh + idx);
-                    dyw[c][0] = d.x; dyw[c][1] = d.y; dyw[c][2] = d.z; dyw[c][3] = d.w;
-                } else {
-                    const float4 ym = ld4(wc + rym), yp = ld4(wc + ryp);
-                    dyw[c][0] = (yp.x - ym.x) * a.k2;
-                    dyw[c][1] = (yp.y - ym.y) * a.k2;
-                    dyw[c][2] = (yp.z - ym.z) * a.k2;
-                    dyw[c][3] = (yp.w - ym.w) * a.k2;
-                }
-                const float4 zm = ld4(wc + rzm), zp = ld4(wc + rzp);
-                dzw[c][0] = (zp.x - zm.x) * kz;
-                dzw[c][1] = (zp.y - zm.y) * kz;
-                dzw[c][2] = (zp.z - zm.z) * kz;
-                dzw[c][3] = (zp.w - zm.w) * kz;
+        for (int c = 0; c < 6; c++)
+            st4(a.tau + c * nh + idx, make_float4(tn[c][0], tn[c][1], tn[c][2], tn[c][3]));
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            amp_m += (double)sqrtf(qm[j] * 0.5f);
+            amp_t += (double)sqrtf(qt[j] * 0.5f);
+        }
+    }
+
+    // Hooke's law (src/elastic3d.f90:129-142) on the strain of w at 4
+    // points; h = C:E is added to the base stress below
+    float h[6][4];
+    if (MODE != MODE_EIGEN) {
+        float dxw[3][4], dyw[3][4], dzw[3][4];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            const float *wc = a.w + c * nh;
+            if (FIR) {
+                const float4 d = ld4(a.wx + c * nh + idx);
+                dxw[c][0] = d.x; dxw[c][1] = d.y; dxw[c][2] = d.z; dxw[c][3] = d.w;
+            } else {
+                const float4 cv = ld4(wc + idx);
+                const float lft = __ldg(wc + row + i1m), rgt = __ldg(wc + row + i1p);
+                dxw[c][0] = (cv.y - lft) * a.k1;
+                dxw[c][1] = (cv.z - cv.x) * a.k1;
+                dxw[c][2] = (cv.w - cv.y) * a.k1;
+                dxw[c][3] = (rgt - cv.z) * a.k1;
+            }
+            if (FIR) {
+                const float4 d = ld4(a.wy + c * nh + idx);
+                dyw[c][0] = d.x; dyw[c][1] = d.y; dyw[c][2] = d.z; dyw[c][3] = d.w;
+            } else {
+                const float4 ym = ld4(wc + rym), yp = ld4(wc + ryp);
+                dyw[c][0] = (yp.x - ym.x) * a.k2;
+                dyw[c][1] = (yp.y - ym.y) * a.k2;
+                dyw[c][2] = (yp.z - ym.z) * a.k2;
+                dyw[c][3] = (yp.w - ym.w) * a.k2;
+            }
+            const float4 zm = ld4(wc + rzm), zp = ld4(wc + rzp);
+            dzw[c][0] = (zp.x - zm.x) * kz;
+            dzw[c][1] = (zp.y - zm.y) * kz;
+            dzw[c][2] = (zp.z - zm.z) * kz;
+            dzw[c][3] = (zp.w - zm.w) * kz;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float e11 = dxw[0][j];
+            const float e12 = (dxw[1][j] + dyw[0][j]) * 0.5f;
+            const float e13 = (dxw[2][j] + dzw[0][j]) * 0.5f;
+            const float e22 = dyw[1][j];
+            const float e23 = (dyw[2][j] + dzw[1][j]) * 0.5f;
+            const float e33 = dzw[2][j];
+            const float tr = e11 + e22 + e33;
+            h[0][j] = a.mu2 * e11 + a.lam * tr;
+            h[1][j] = a.mu2 * e12;
+            h[2][j] = a.mu2 * e13;
+            h[3][j] = a.mu2 * e22 + a.lam * tr;
+            h[4][j] = a.mu2 * e23;
+            h[5][j] = a.mu2 * e33 + a.lam * tr;
+        }
+    }
+
+    // base stress + h.  Tensor amplitudes (tensornorm, weights 1 2 2 1 2 1
+    // over the components) accumulate one component at a time.
+    float s[6][4];
+    constexpr float wnorm[6] = {1.f, 2.f, 2.f, 1.f, 2.f, 1.f};
+    if (MODE == MODE_OP) {
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            const float4 v = ldc4(a.sig + c * nh + idx);
+            s[c][0] = v.x + h[c][0]; s[c][1] = v.y + h[c][1]; s[c][2] = v.z + h[c][2]; s[c][3] = v.w + h[c][3];
+        }
+    } else if (MODE == MODE_EIGEN) {
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            const float4 v = ldc4(a.sig + c * nh + idx);
+            s[c][0] = v.x; s[c][1] = v.y; s[c][2] = v.z; s[c][3] = v.w;
+        }
+    } else if (MODE == MODE_INIT) {
+        float qt[4];
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            const float4 t = src.tau(a, c, idx);
+            const float tv[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                qt[j] = c == 0 ? tv[j] * tv[j] : qt[j] + wnorm[c] * tv[j] * tv[j];
+                s[c][j] = -tv[j] + h[c][j];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) amp_t += (double)sqrtf(qt[j] * 0.5f);
+    } else if (MODE == MODE_END) {
+#pragma unroll
+        for (int c = 0; c < 6; c++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) s[c][j] = -tn[c][j] + h[c][j];
+    } else {  // MODE_CORR
+        const float c1 = -(float)(a.st->Dt / 2);
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            const float4 t = src.tau(a, c, idx);
+            const float4 m = src.m(a, c, idx);
+            s[c][0] = (c1 * m.x - t.x) + h[c][0]; s[c][1] = (c1 * m.y - t.y) + h[c][1];
+            s[c][2] = (c1 * m.z - t.z) + h[c][2]; s[c][3] = (c1 * m.w - t.w) + h[c][3];
+        }
+    }
+    if (keep) {
+#pragma unroll
+        for (int c = 0; c < 6; c++)
+            st4(a.sig + c * nh + idx, make_float4(s[c][0], s[c][1], s[c][2], s[c][3]));
+    }
+
+    if (MODE != MODE_OP) {
+        // viscouseigenstress for the linear and power-law mechanisms
+        float mo[6][4];
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (MODE == MODE_EIGEN) v = src.m(a, c, idx);
+            mo[c][0] = v.x; mo[c][1] = v.y; mo[c][2] = v.z; mo[c][3] = v.w;
+        }
+        float sp[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (a.spdev) {
+#pragma unroll
+            for (int c = 0; c < 6; c++) sp[c] = __ldg(a.spdev + c * g.sx3h + i3);
+        }
+        float gsum[4] = {0.f, 0.f, 0.f, 0.f};
+        const float dtf = MODE == MODE_CORR ? (float)a.st->Dt : 0.f;
+        float4 gold = make_float4(0.f, 0.f, 0.f, 0.f);
+        if ((MODE == MODE_CORR || MODE == MODE_EIGEN) && a.gamma) gold = ldc4(a.gamma + idx);
+        float gacc[4] = {gold.x, gold.y, gold.z, gold.w};
+        // the largest gammadot per mechanism: its reciprocal is the
+        // minimum of the points' 1/gammadot (a correctly rounded
+        // reciprocal is monotonic), one division instead of four
+        float gmx[2] = {0.f, 0.f};
+#pragma unroll
+        for (int mech = 0; mech < 2; mech++) {
+            if (!a.visc[mech]) continue;
+            const DepthVisc dv = a.visc[mech][i3];
+            float g0v[4] = {dv.g0, dv.g0, dv.g0, dv.g0};
+            if (a.dg0[mech]) {
+                const float4 d = ld4(a.dg0[mech] + idx);
+                g0v[0] += d.x; g0v[1] += d.y; g0v[2] += d.z; g0v[3] += d.w;
             }
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const float e11 = dxw[0][j];
-                const float e12 = (dxw[1][j] + dyw[0][j]) * 0.5f;
-                const float e13 = (dxw[2][j] + dzw[0][j]) * 0.5f;
-                const float e22 = dyw[1][j];
-                const float e23 = (dyw[2][j] + dzw[1][j]) * 0.5f;
-                const float e33 = dzw[2][j];
-                const float tr = e11 + e22 + e33;
-                h[0][j] = a.mu2 * e11 + a.lam * tr;
-                h[1][j] = a.mu2 * e12;
-                h[2][j] = a.mu2 * e13;
-                h[3][j] = a.mu2 * e22 + a.lam * tr;
-                h[4][j] = a.mu2 * e23;
-                h[5][j] = a.mu2 * e33 + a.lam * tr;
+                gsum[j] = 0.f;
+                if (!(g0v[j] >= 1.0e-20f)) continue;
+                const float tr3 = (s[0][j] + s[3][j] + s[5][j]) * (1.f / 3.f);
+                const float d11 = s[0][j] - tr3, d22 = s[3][j] - tr3, d33 = s[5][j] - tr3;
+                const float tau = tnorm6(d11 + sp[0], s[1][j] + sp[1], s[2][j] + sp[2],
+                                         d22 + sp[3], s[4][j] + sp[4], d33 + sp[5]);
+                const float tauc = fmaxf(0.f, tau - dv.cohesion);
+                if (!(tauc > 1.0e-20f)) continue;
+                const float x = tauc * a.muinv;
+                const float pe = dv.power - 1.f;
+                float gd;
+                if (pe == 0.f) gd = g0v[j];
+                else if (pe == 1.f) gd = g0v[j] * x;
+                else if (pe == 2.f) gd = g0v[j] * x * x;
+                else gd = g0v[j] * powf(x, pe);
+                const float gd2 = 2.f * gd, gp2 = 2.f * g0v[j] * dv.tpow;
+                mo[0][j] += gd2 * d11 - gp2 * sp[0];
+                mo[1][j] += gd2 * s[1][j] - gp2 * sp[1];
+                mo[2][j] += gd2 * s[2][j] - gp2 * sp[2];
+                mo[3][j] += gd2 * d22 - gp2 * sp[3];
+                mo[4][j] += gd2 * s[4][j] - gp2 * sp[4];
+                mo[5][j] += gd2 * d33 - gp2 * sp[5];
+                gmx[mech] = fmaxf(gmx[mech], gd);
+                gsum[j] = gd * x;
+                if (MODE == MODE_EIGEN) gacc[j] = gsum[j];
+            }
+            if (MODE == MODE_CORR) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) gacc[j] = gacc[j] + dtf * gsum[j];
             }
         }
-
-        // base stress + h.  Tensor amplitudes (tensornorm, weights 1 2 2 1 2 1
-        // over the components) accumulate one component at a time.
-        float s[6][4];
-        constexpr float wnorm[6] = {1.f, 2.f, 2.f, 1.f, 2.f, 1.f};
-        if (MODE == MODE_OP) {
+#pragma unroll
+        for (int mech = 0; mech < 2; mech++) tmin[mech] = fminf(tmin[mech], 1.f / gmx[mech]);
+        if (TRANS && (MODE == MODE_INIT || MODE == MODE_END || MODE == MODE_CORR) && a.eps) {
+            float ep[6][4], in[6][4], rate[6][4];
 #pragma unroll
             for (int c = 0; c < 6; c++) {
-                const float4 v = ldc4(a.sig + c * nh + idx);
-                s[c][0] = v.x + h[c][0]; s[c][1] = v.y + h[c][1]; s[c][2] = v.z + h[c][2]; s[c][3] = v.w + h[c][3];
+                const float4 e = ldc4(a.eps + c * nh + idx);
+                ep[c][0] = e.x; ep[c][1] = e.y; ep[c][2] = e.z; ep[c][3] = e.w;
             }
-        } else if (MODE == MODE_EIGEN) {
+            if (MODE == MODE_CORR) {
+                const float h = (float)(a.st->Dt / 2);
 #pragma unroll
-            for (int c = 0; c < 6; c++) {
-                const float4 v = ldc4(a.sig + c * nh + idx);
-                s[c][0] = v.x; s[c][1] = v.y; s[c][2] = v.z; s[c][3] = v.w;
-            }
-        } else if (MODE == MODE_INIT) {
-            float qt[4];
-#pragma unroll
-            for (int c = 0; c < 6; c++) {
-                const float4 t = ldc4(a.tau + c * nh + idx);
-                const float tv[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    qt[j] = c == 0 ? tv[j] * tv[j] : qt[j] + wnorm[c] * tv[j] * tv[j];
-                    s[c][j] = -tv[j] + h[c][j];
+                for (int c = 0; c < 6; c++) {
+                    const float4 r = ldc4(a.epsdot + c * nh + idx);
+                    in[c][0] = h * r.x + ep[c][0]; in[c][1] = h * r.y + ep[c][1];
+                    in[c][2] = h * r.z + ep[c][2]; in[c][3] = h * r.w + ep[c][3];
                 }
-            }
+            } else {
 #pragma unroll
-            for (int j = 0; j < 4; j++) amp_t += (double)sqrtf(qt[j] * 0.5f);
-        } else if (MODE == MODE_END) {
+                for (int c = 0; c < 6; c++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) in[c][j] = ep[c][j];
+            }
 #pragma unroll
             for (int c = 0; c < 6; c++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) s[c][j] = -tn[c][j] + h[c][j];
-        } else {  // MODE_CORR
-            const float c1 = -(float)(a.st->Dt / 2);
+                for (int j = 0; j < 4; j++) rate[c][j] = 0.f;
 #pragma unroll
-            for (int c = 0; c < 6; c++) {
-                const float4 t = ldc4(a.tau + c * nh + idx);
-                const float4 m = ldc4(a.m + c * nh + idx);
-                s[c][0] = (c1 * m.x - t.x) + h[c][0]; s[c][1] = (c1 * m.y - t.y) + h[c][1];
-                s[c][2] = (c1 * m.z - t.z) + h[c][2]; s[c][3] = (c1 * m.w - t.w) + h[c][3];
-            }
-        }
-        if (MODE == MODE_OP || (MODE != MODE_EIGEN && a.store_sig && (!a.sig_mask || a.sig_mask[q]))) {
-#pragma unroll
-            for (int c = 0; c < 6; c++)
-                st4(a.sig + c * nh + idx, make_float4(s[c][0], s[c][1], s[c][2], s[c][3]));
-        }
-
-        if (MODE != MODE_OP) {
-            // viscouseigenstress for the linear and power-law mechanisms
-            float mo[6][4];
-#pragma unroll
-            for (int c = 0; c < 6; c++) {
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (MODE == MODE_EIGEN) v = ldc4(a.m + c * nh + idx);
-                mo[c][0] = v.x; mo[c][1] = v.y; mo[c][2] = v.z; mo[c][3] = v.w;
-            }
-            float sp[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            if (a.spdev) {
-#pragma unroll
-                for (int c = 0; c < 6; c++) sp[c] = __ldg(a.spdev + c * g.sx3h + i3);
-            }
-            float gsum[4] = {0.f, 0.f, 0.f, 0.f};
-            const float dtf = MODE == MODE_CORR ? (float)a.st->Dt : 0.f;
-            float4 gold = make_float4(0.f, 0.f, 0.f, 0.f);
-            if ((MODE == MODE_CORR || MODE == MODE_EIGEN) && a.gamma) gold = ldc4(a.gamma + idx);
-            float gacc[4] = {gold.x, gold.y, gold.z, gold.w};
-            // the largest gammadot per mechanism: its reciprocal is the
-            // minimum of the points' 1/gammadot (a correctly rounded
-            // reciprocal is monotonic), one division instead of four
-            float gmx[2] = {0.f, 0.f};
-#pragma unroll
-            for (int mech = 0; mech < 2; mech++) {
-                if (!a.visc[mech]) continue;
-                const DepthVisc dv = a.visc[mech][i3];
-                float g0v[4] = {dv.g0, dv.g0, dv.g0, dv.g0};
-                if (a.dg0[mech]) {
-                    const float4 d = ld4(a.dg0[mech] + idx);
+            for (int tm = 0; tm < 2; tm++) {
+                if (!a.trans[tm]) continue;
+                const TransLayer L = a.trans[tm][i3];
+                float g0v[4] = {L.g0, L.g0, L.g0, L.g0};
+                if (a.tdg0[tm]) {
+                    const float4 d = ld4(a.tdg0[tm] + idx);
                     g0v[0] += d.x; g0v[1] += d.y; g0v[2] += d.z; g0v[3] += d.w;
                 }
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
-                    gsum[j] = 0.f;
-                    if (!(g0v[j] >= 1.0e-20f)) continue;
+#pragma unroll
+                    for (int c = 0; c < 6; c++) rate[c][j] = 0.f;
+                    if (1.0e-20f > g0v[j]) continue;
                     const float tr3 = (s[0][j] + s[3][j] + s[5][j]) * (1.f / 3.f);
-                    const float d11 = s[0][j] - tr3, d22 = s[3][j] - tr3, d33 = s[5][j] - tr3;
-                    const float tau = tnorm6(d11 + sp[0], s[1][j] + sp[1], s[2][j] + sp[2],
-                                             d22 + sp[3], s[4][j] + sp[4], d33 + sp[5]);
-                    const float tauc = fmaxf(0.f, tau - dv.cohesion);
-                    if (!(tauc > 1.0e-20f)) continue;
-                    const float x = tauc * a.muinv;
-                    const float pe = dv.power - 1.f;
+                    // Q = s' - 2 Gk epsilonik
+                    const float Q[6] = {(s[0][j] - tr3) - L.gk2 * in[0][j], s[1][j] - L.gk2 * in[1][j],
+                                        s[2][j] - L.gk2 * in[2][j], (s[3][j] - tr3) - L.gk2 * in[3][j],
+                                        s[4][j] - L.gk2 * in[4][j], (s[5][j] - tr3) - L.gk2 * in[5][j]};
+                    const float x = tnorm6(Q[0], Q[1], Q[2], Q[3], Q[4], Q[5]) * a.muinv;
+                    const float pe = L.power - 1.f;
                     float gd;
                     if (pe == 0.f) gd = g0v[j];
                     else if (pe == 1.f) gd = g0v[j] * x;
                     else if (pe == 2.f) gd = g0v[j] * x * x;
                     else gd = g0v[j] * powf(x, pe);
-                    const float gd2 = 2.f * gd, gp2 = 2.f * g0v[j] * dv.tpow;
-                    mo[0][j] += gd2 * d11 - gp2 * sp[0];
-                    mo[1][j] += gd2 * s[1][j] - gp2 * sp[1];
-                    mo[2][j] += gd2 * s[2][j] - gp2 * sp[2];
-                    mo[3][j] += gd2 * d22 - gp2 * sp[3];
-                    mo[4][j] += gd2 * s[4][j] - gp2 * sp[4];
-                    mo[5][j] += gd2 * d33 - gp2 * sp[5];
-                    gmx[mech] = fmaxf(gmx[mech], gd);
-                    gsum[j] = gd * x;
-                    if (MODE == MODE_EIGEN) gacc[j] = gsum[j];
-                }
-                if (MODE == MODE_CORR) {
-#pragma unroll
-                    for (int j = 0; j < 4; j++) gacc[j] = gacc[j] + dtf * gsum[j];
-                }
-            }
-#pragma unroll
-            for (int mech = 0; mech < 2; mech++) tmin[mech] = fminf(tmin[mech], 1.f / gmx[mech]);
-            if (TRANS && (MODE == MODE_INIT || MODE == MODE_END || MODE == MODE_CORR) && a.eps) {
-                float ep[6][4], in[6][4], rate[6][4];
-#pragma unroll
-                for (int c = 0; c < 6; c++) {
-                    const float4 e = ldc4(a.eps + c * nh + idx);
-                    ep[c][0] = e.x; ep[c][1] = e.y; ep[c][2] = e.z; ep[c][3] = e.w;
-                }
-                if (MODE == MODE_CORR) {
-                    const float h = (float)(a.st->Dt / 2);
+                    const float rq = gd * a.muinv, gd2 = 2.f * gd;
 #pragma unroll
                     for (int c = 0; c < 6; c++) {
-                        const float4 r = ldc4(a.epsdot + c * nh + idx);
-                        in[c][0] = h * r.x + ep[c][0]; in[c][1] = h * r.y + ep[c][1];
-                        in[c][2] = h * r.z + ep[c][2]; in[c][3] = h * r.w + ep[c][3];
+                        rate[c][j] = rq * Q[c];
+                        mo[c][j] += gd2 * Q[c];
                     }
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 6; c++)
-#pragma unroll
-                        for (int j = 0; j < 4; j++) in[c][j] = ep[c][j];
-                }
-#pragma unroll
-                for (int c = 0; c < 6; c++)
-#pragma unroll
-                    for (int j = 0; j < 4; j++) rate[c][j] = 0.f;
-#pragma unroll
-                for (int tm = 0; tm < 2; tm++) {
-                    if (!a.trans[tm]) continue;
-                    const TransLayer L = a.trans[tm][i3];
-                    float g0v[4] = {L.g0, L.g0, L.g0, L.g0};
-                    if (a.tdg0[tm]) {
-                        const float4 d = ld4(a.tdg0[tm] + idx);
-                        g0v[0] += d.x; g0v[1] += d.y; g0v[2] += d.z; g0v[3] += d.w;
-                    }
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-#pragma unroll
-                        for (int c = 0; c < 6; c++) rate[c][j] = 0.f;
-                        if (1.0e-20f > g0v[j]) continue;
-                        const float tr3 = (s[0][j] + s[3][j] + s[5][j]) * (1.f / 3.f);
-                        // Q = s' - 2 Gk epsilonik
-                        const float Q[6] = {(s[0][j] - tr3) - L.gk2 * in[0][j], s[1][j] - L.gk2 * in[1][j],
-                                            s[2][j] - L.gk2 * in[2][j], (s[3][j] - tr3) - L.gk2 * in[3][j],
-                                            s[4][j] - L.gk2 * in[4][j], (s[5][j] - tr3) - L.gk2 * in[5][j]};
-                        const float x = tnorm6(Q[0], Q[1], Q[2], Q[3], Q[4], Q[5]) * a.muinv;
-                        const float pe = L.power - 1.f;
-                        float gd;
-                        if (pe == 0.f) gd = g0v[j];
-                        else if (pe == 1.f) gd = g0v[j] * x;
-                        else if (pe == 2.f) gd = g0v[j] * x * x;
-                        else gd = g0v[j] * powf(x, pe);
-                        const float rq = gd * a.muinv, gd2 = 2.f * gd;
-#pragma unroll
-                        for (int c = 0; c < 6; c++) {
-                            rate[c][j] = rq * Q[c];
-                            mo[c][j] += gd2 * Q[c];
-                        }
-                        if (MODE != MODE_CORR) tmin[2 + tm] = fminf(tmin[2 + tm], 1.f / gd);
-                    }
-                    if (MODE == MODE_CORR) {
-                        // the corrector's next call reads epsilonikdot, i.e. this rate
-#pragma unroll
-                        for (int c = 0; c < 6; c++)
-#pragma unroll
-                            for (int j = 0; j < 4; j++) in[c][j] = rate[c][j];
-                    }
+                    if (MODE != MODE_CORR) tmin[2 + tm] = fminf(tmin[2 + tm], 1.f / gd);
                 }
                 if (MODE == MODE_CORR) {
+                    // the corrector's next call reads epsilonikdot, i.e. this rate
 #pragma unroll
                     for (int c = 0; c < 6; c++)
-                        st4(a.eps + c * nh + idx,
-                            make_float4(ep[c][0] + dtf * rate[c][0], ep[c][1] + dtf * rate[c][1],
-                                        ep[c][2] + dtf * rate[c][2], ep[c][3] + dtf * rate[c][3]));
-                } else {
 #pragma unroll
-                    for (int c = 0; c < 6; c++)
-                        st4(a.epsdot + c * nh + idx, make_float4(rate[c][0], rate[c][1], rate[c][2], rate[c][3]));
+                        for (int j = 0; j < 4; j++) in[c][j] = rate[c][j];
                 }
             }
+            if (MODE == MODE_CORR) {
 #pragma unroll
-            for (int c = 0; c < 6; c++)
-                st4(a.m + c * nh + idx, make_float4(mo[c][0], mo[c][1], mo[c][2], mo[c][3]));
-            if ((MODE == MODE_CORR || MODE == MODE_EIGEN) && a.gamma)
-                st4(a.gamma + idx, make_float4(gacc[0], gacc[1], gacc[2], gacc[3]));
+                for (int c = 0; c < 6; c++)
+                    st4(a.eps + c * nh + idx,
+                        make_float4(ep[c][0] + dtf * rate[c][0], ep[c][1] + dtf * rate[c][1],
+                                    ep[c][2] + dtf * rate[c][2], ep[c][3] + dtf * rate[c][3]));
+            } else {
+#pragma unroll
+                for (int c = 0; c < 6; c++)
+                    st4(a.epsdot + c * nh + idx, make_float4(rate[c][0], rate[c][1], rate[c][2], rate[c][3]));
+            }
         }
+#pragma unroll
+        for (int c = 0; c < 6; c++)
+            st4(a.m + c * nh + idx, make_float4(mo[c][0], mo[c][1], mo[c][2], mo[c][3]));
+        if ((MODE == MODE_CORR || MODE == MODE_EIGEN) && a.gamma)
+            st4(a.gamma + idx, make_float4(gacc[0], gacc[1], gacc[2], gacc[3]));
     }
+}
 
+// The block reductions of a stress pass: per-block partials and, with a
+// ticket, their reduction by the last block.  All threads call.
+template <int MODE, bool TRANS>
+__device__ __forceinline__ void stress_reduce(const StressArgs &a, const float (&tmin)[4], double amp_m, double amp_t)
+{
+    constexpr int NTM = TRANS ? 4 : 2;        // Maxwell-time minima: viscous 2 (+ transient 2)
+    __shared__ float shf[32];
+    __shared__ double shd[32];
     if (MODE == MODE_INIT || MODE == MODE_END || MODE == MODE_EIGEN) {
         // the block reductions in one pass (fixed order, one barrier); 8 warps
         float tq[4];
@@ -608,6 +620,100 @@ __global__ void __launch_bounds__(RELAX_NTHREADS, TRANS ? 2 : 3) k_stress(const 
             }
         }
     }
+}
+
+template <int MODE, bool BATCH = false, bool TRANS = false, bool FIR = false>
+__global__ void __launch_bounds__(RELAX_NTHREADS, TRANS ? 2 : 3) k_stress(const __grid_constant__ StressArgs a0)
+{
+    pdl_enter();
+    const StressArgs &a = BATCH ? a0.tab[blockIdx.y] : a0;
+    if (MODE == MODE_END && a.st->fire) return;   // the event branch of the step runs instead
+    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    float tmin[4] = {3.0e38f, 3.0e38f, 3.0e38f, 3.0e38f};
+    double amp_m = 0.0, amp_t = 0.0;
+    if (q < a.g.nh >> 2) stress_group<MODE, TRANS, FIR>(a, q, FromGlobal{}, tmin, amp_m, amp_t);
+    stress_reduce<MODE, TRANS>(a, tmin, amp_m, amp_t);
+}
+
+// The END pass with tau and m, four fifths of what it reads, brought in by
+// bulk copies: SP_STAGES tiles of 256 groups in shared memory, SP_BLOCKS
+// persistent blocks an SM that take the tiles in turn.  With loads into
+// registers alone (24 warps an SM, two waits a group) the memory was idle
+// between the waits: 108 -> 95 us on the 256 x 256 x 128 box, 762 -> 659 us
+// (84 % of the copy bandwidth) on 512 x 512 x 256, 189 -> 158 us on 256^3.
+// Tiles of 128 groups and 4 blocks measured 710 us on the large box, the
+// strain ahead of the wait 96 us on the first, and the CORR pass in this form
+// 81 us against 71 (its stencil loads, not tau and m, are what it waits for).
+constexpr int SP_STAGES = 2, SP_BLOCKS = 2, SP_TILE = RELAX_NTHREADS;
+constexpr size_t SP_SMEM = (size_t)SP_STAGES * 12 * SP_TILE * sizeof(float4);
+
+template <bool BATCH = false>
+__global__ void __launch_bounds__(SP_TILE, SP_BLOCKS) k_stress_pipe(const __grid_constant__ StressArgs a0)
+{
+    pdl_enter();
+    const StressArgs &a = BATCH ? a0.tab[blockIdx.y] : a0;
+    if (a.st->fire) return;   // the event branch of the step runs instead
+    extern __shared__ __align__(128) float4 tiles[];   // [SP_STAGES][12][SP_TILE]
+    __shared__ __align__(8) uint64_t full[SP_STAGES];
+    const size_t nq = a.g.nh >> 2, nh = a.g.nh;
+    const int ntile = (int)((nq + SP_TILE - 1) / SP_TILE);
+    auto bar = [&](int s) { return async::smem_u32(&full[s]); };
+    auto issue = [&](int tile, int s) {
+        const size_t q0 = (size_t)tile * SP_TILE;
+        const uint32_t bytes = (uint32_t)min((size_t)SP_TILE, nq - q0) * sizeof(float4);
+        async::mbar_expect(bar(s), 12 * bytes);
+        for (int c = 0; c < 12; c++)
+            async::bulk_load(async::smem_u32(tiles + (s * 12 + c) * SP_TILE), (c < 6 ? a.tau + c * nh : a.m + (c - 6) * nh) + 4 * q0,
+                             bytes, bar(s));
+    };
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < SP_STAGES; s++) async::mbar_init(bar(s), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int s = 0; s < SP_STAGES; s++)
+            if ((int)(blockIdx.x + s * gridDim.x) < ntile) issue(blockIdx.x + s * gridDim.x, s);
+    float tmin[4] = {3.0e38f, 3.0e38f, 3.0e38f, 3.0e38f};
+    double amp_m = 0.0, amp_t = 0.0;
+    int s = 0, ph = 0;
+    for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+        const bool ok = async::mbar_wait(bar(s), ph);
+        FromRegs src;
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            src.t[c] = tiles[(s * 12 + c) * SP_TILE + threadIdx.x];
+            src.v[c] = tiles[(s * 12 + 6 + c) * SP_TILE + threadIdx.x];
+        }
+        if (__syncthreads_or(!ok)) {
+            // a copy that never came: report it, wait (again with a limit)
+            // for those still in flight, and leave
+            if (threadIdx.x == 0) {
+                atomicOr(a.err, 1 << RELAX_ERR_CUDA);
+                for (int r = 1; r < SP_STAGES; r++) {
+                    const int o = (s + r) % SP_STAGES;
+                    if (tile + (int)(r * gridDim.x) < ntile) async::mbar_wait(bar(o), o < s ? ph ^ 1 : ph);
+                }
+            }
+            __syncthreads();
+            return;
+        }
+        const size_t q = (size_t)tile * SP_TILE + threadIdx.x;
+        if (q < nq) stress_group<MODE_END, false, false>(a, q, src, tmin, amp_m, amp_t);
+        // The next tile into this one's place once every thread has used its
+        // values (stored tau and m): a copy set off right after the reads can
+        // overtake the reads that still wait in a warp's queue, which a
+        // barrier alone does not drain.
+        async::fence_reads();
+        __syncthreads();
+        const int next = tile + SP_STAGES * gridDim.x;
+        if (threadIdx.x == 0 && next < ntile) issue(next, s);
+        if (++s == SP_STAGES) {
+            s = 0;
+            ph ^= 1;
+        }
+    }
+    stress_reduce<MODE_END, false>(a, tmin, amp_m, amp_t);
 }
 
 // tau += Dt m with the amplitude of m (coseismic-event path of the step,

@@ -1081,11 +1081,25 @@ static StressArgs stress_args(relax_ctx *c, const float *w)
     a.ticket = c->ticket;
     a.fin = c->dst;
     a.dv = g.dx1 * g.dx2 * g.dx3;
+    a.err = c->err;
     for (int k = 0; k < 2; k++) { a.trans[k] = c->tvisc[k]; a.tdg0[k] = c->tdg0[k]; }
     a.eps = c->eps; a.epsdot = c->epsdot;
     a.tm_part = c->tm_part;
     a.amp_part = c->amp_part;
     return a;
+}
+
+// The pipelined form of the END pass, where each of its blocks has at least
+// two tiles (smaller boxes have no next tile to fetch).  The grid is a
+// function of the box alone, so that a batch reduces in the order of a member
+// stepped by itself.
+constexpr int kPipeBlocks = 148 * SP_BLOCKS;
+static bool pipe_ok(const Grid &g) { return (int)nblocks(g.nh / 4, SP_TILE) >= 2 * kPipeBlocks; }
+template <bool BATCH>
+static void launch_stress_pipe(const StressArgs &a, int nm, cudaStream_t st)
+{
+    set_smem(k_stress_pipe<BATCH>, SP_SMEM);
+    launch_pdl(k_stress_pipe<BATCH>, dim3(kPipeBlocks, nm), SP_TILE, SP_SMEM, st, a);
 }
 
 template <int MODE>
@@ -1115,6 +1129,8 @@ static int launch_stress(relax_ctx *c, StressArgs a)
     }
     if (trans)
         TIMED(&c->prof, stage, c->st, (launch_pdl(k_stress<MODE, false, true>, c->nblk, RELAX_NTHREADS, 0, c->st, a)));
+    else if (MODE == MODE_END && pipe_ok(c->g))
+        TIMED(&c->prof, stage, c->st, (launch_stress_pipe<false>(a, 1, c->st)));
     else
         TIMED(&c->prof, stage, c->st, (launch_pdl(k_stress<MODE>, c->nblk, RELAX_NTHREADS, 0, c->st, a)));
     return RELAX_OK;
@@ -1721,8 +1737,10 @@ static int check_err(relax_ctx *c)
 {
     if (c->hst->error & (1 << RELAX_ERR_FRICTION))
         return fail(RELAX_ERR_FRICTION, "wrong value of (a-b)sigma: tau/((a-b)sigma) > 20");
-    if (c->hst->error & (1 << RELAX_ERR_CUDA))
-        return fail(RELAX_ERR_CUDA, "tensor-core x3 pass: a wait on the tensor cores timed out");
+    if (c->hst->error & (1 << RELAX_ERR_CUDA)) {
+        cudaMemsetAsync(c->ticket, 0, sizeof(unsigned), c->st);   // the pass that gave up did not count its blocks out
+        return fail(RELAX_ERR_CUDA, "the x3 pass on the tensor cores or a stress pass: a wait on an asynchronous operation timed out");
+    }
     return RELAX_OK;
 }
 
@@ -1827,7 +1845,7 @@ static int finish_step(relax_ctx *c, relax_step_log *log)
             output = 1;
         }
     }
-    if (!c->fc.empty()) TRY(check_err(c));
+    TRY(check_err(c));
     log->i = c->i;
     log->event = fired;
     log->dt = Dt;
@@ -3593,6 +3611,7 @@ static int batch_kernels(relax_batch *b)
     CKL();
     TRY(batch_green(b, t.xic0));
     if (b->trans) launch_pdl(k_stress<MODE_END, true, true>, dim3(c0->nblk, n), RELAX_NTHREADS, 0, st, t.end0);
+    else if (pipe_ok(c0->g)) launch_stress_pipe<true>(t.end0, n, st);
     else launch_pdl(k_stress<MODE_END, true>, dim3(c0->nblk, n), RELAX_NTHREADS, 0, st, t.end0);
     b->launches++;
     CKL();

@@ -37,7 +37,8 @@
 namespace relax {
 namespace tc {
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+using namespace async;
+
 
 // Shared-memory matrix descriptor of an operand in the no-swizzle canonical
 // layout: 8 rows x 16 bytes core matrices; lbo / sbo the byte strides of the
@@ -79,31 +80,6 @@ __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::be
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 // generic-proxy shared-memory writes made visible to the tensor cores
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-// bounded wait for the phase `parity` of an mbarrier to complete
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
-{
-    for (int it = 0; it < (1 << 22); it++)
-        if (mbar_try(bar, parity)) return true;
-    return false;
-}
 
 // 32 lanes x 32 columns of FP32 from tensor memory (lane = row of the warp's
 // quarter, one column per register) and back
