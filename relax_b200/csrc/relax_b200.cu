@@ -2817,9 +2817,9 @@ extern "C" int relax_op_bodyforce(const relax_tensor *sig, double dx1, double dx
     float *s;
     TRY(sc.get(&s, 6 * g.nh));
     k_aos_to_soa<<<nblocks(g.nh), RELAX_NTHREADS, 0, st>>>(sig, s, g.nh);
-    k_bodyforce<<<nblocks(g.nh), RELAX_NTHREADS, 0, st>>>(g, s, c1, c2, c3, t1, t2, t3, (float)(0.5 / dx1),
-                                                          (float)(0.5 / dx2), (float)(0.5 / dx3), (float)(1.0 / dx3),
-                                                          fir_x(g), fir_y(g));
+    auto k = has_fir(g) ? k_bodyforce<true> : k_bodyforce<false>;
+    k<<<nblocks(g.nh), RELAX_NTHREADS, 0, st>>>(g, s, c1, c2, c3, t1, t2, t3, (float)(0.5 / dx1), (float)(0.5 / dx2),
+                                                (float)(0.5 / dx3), (float)(1.0 / dx3), fir_x(g), fir_y(g));
     CKL();
     return RELAX_OK;
 }

@@ -327,42 +327,59 @@ __global__ void __launch_bounds__(CW *N1, zblocks(N1 *N2, N1, CW)) k_zpass(const
 //     F = sum_m fi cos(2 pi m i3 / n),  G = sum_m fi g sin(2 pi m i3 / n)
 // over the wavenumbers m of x3, fi = 2 beta / ((2 pi k3)^2 + beta^2), g = 2
 // pi k3 fi, summed in FP64; two columns in one entry (F, F, G, G).  A block
-// takes 16 columns of one row.
+// takes 16 columns of one row.  The sums over even and odd m for i3 give
+// n/2 - i3 as well (cos and sin of pi m - x), and n - i3 by symmetry: a
+// quarter of the sums.  Bound by FP64 arithmetic and shared memory: 128 x 128
+// x 128 in 17.5 us (48 with a sum for every plane).
 constexpr int ZT_CW = 16;
 __global__ void __launch_bounds__(256) k_ztable(Grid g, float4 *fg, size_t fgs, int planes, double ik1, double ik2,
                                                 double ik3)
 {
     extern __shared__ double zs[];
     const int n = g.sx3, h = n / 2;
-    double *ct = zs, *f = zs + n, *fgn = f + ZT_CW * (h + 1);   // cos table, fi and fi g by (m, column)
+    double2 *cs = reinterpret_cast<double2 *>(zs);                 // cos, sin of 2 pi j / n
+    double2 *f = cs + n;                                           // fi, fi g by (m, column)
     const double PI2 = 6.28318530717958623199592693708837032318;
     const int k1b = ZT_CW * blockIdx.x, k2 = blockIdx.y;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) ct[j] = cospi(2.0 * j / n);
+    for (int j = threadIdx.x; j < n; j += blockDim.x) sincospi(2.0 * j / n, &cs[j].y, &cs[j].x);
     for (int s = threadIdx.x; s < ZT_CW * (h + 1); s += blockDim.x) {
         const int m = s / ZT_CW, k1 = k1b + s % ZT_CW;
         const double k1v = k1 * ik1, k2v = k2 * ik2, b2 = PI2 * PI2 * (k1v * k1v + k2v * k2v);
         const double k3 = PI2 * m * ik3, fi = b2 > 0.0 ? 2.0 * sqrt(b2) / (k3 * k3 + b2) : 0.0;
-        f[s] = fi;
-        fgn[s] = k3 * fi * fi;
+        f[s] = make_double2(fi, k3 * fi * fi);
     }
     __syncthreads();
     const int col = threadIdx.x % ZT_CW, k1 = k1b + col;
     if (k1 >= g.KP) return;
-    for (int z = threadIdx.x / ZT_CW; z < planes; z += blockDim.x / ZT_CW) {
-        double F = f[col] + (z & 1 ? -1.0 : 1.0) * f[h * ZT_CW + col], G = 0.0;
+    auto put = [&](int z, double F, double G) {
+        if (z >= planes) return;
+        float *o = reinterpret_cast<float *>(fg + z * fgs + (size_t)k2 * (g.KP / 2) + k1 / 2);
+        o[k1 & 1] = (float)F;
+        o[2 + (k1 & 1)] = (float)G;
+    };
+    for (int z = threadIdx.x / ZT_CW; z <= n / 4; z += blockDim.x / ZT_CW) {
+        // even and odd wavenumbers; the first and the last stand alone
+        double F[2] = {0.5 * f[col].x, 0.0}, G[2] = {0.0, 0.0};
+        F[h & 1] += 0.5 * (z & 1 ? -1.0 : 1.0) * f[h * ZT_CW + col].x;
         int j = 0;   // m z mod n
         for (int m = 1; m < h; m++) {
             j += z;
             if (j >= n) j -= n;
-            int q = j - n / 4;   // sin x = cos(x - pi/2) where n is a multiple of 4
-            if (q < 0) q += n;
-            const double sn = n % 4 ? sinpi(2.0 * j / n) : ct[q];
-            F += 2.0 * f[m * ZT_CW + col] * ct[j];
-            G += 2.0 * fgn[m * ZT_CW + col] * sn;
+            const double2 t = cs[j], v = f[m * ZT_CW + col];
+            if (m & 1) {
+                F[1] += v.x * t.x;
+                G[1] += v.y * t.y;
+            } else {
+                F[0] += v.x * t.x;
+                G[0] += v.y * t.y;
+            }
         }
-        float *o = reinterpret_cast<float *>(fg + z * fgs + (size_t)k2 * (g.KP / 2) + k1 / 2);
-        o[k1 & 1] = (float)F;
-        o[2 + (k1 & 1)] = (float)G;
+        const double Fz = 2.0 * (F[0] + F[1]), Gz = 2.0 * (G[0] + G[1]);
+        const double Fh = 2.0 * (F[0] - F[1]), Gh = 2.0 * (G[1] - G[0]);
+        put(z, Fz, Gz);
+        put(h - z, Fh, Gh);
+        if (z) put(n - z, Fz, -Gz);
+        put(h + z, Fh, -Gh);
     }
 }
 
@@ -387,7 +404,7 @@ size_t zspec_table_stride(const Grid &g) { return (size_t)(g.sx2 - g.sx2 / 2 + 1
 
 cudaError_t zspec_table(const Grid &g, float4 *fg, int planes, cudaStream_t st)
 {
-    const size_t sm = (g.sx3 + 2 * ZT_CW * (size_t)(g.sx3 / 2 + 1)) * sizeof(double);
+    const size_t sm = (g.sx3 + ZT_CW * (size_t)(g.sx3 / 2 + 1)) * sizeof(double2);
     set_smem(k_ztable, sm);
     const dim3 grid((g.KP + ZT_CW - 1) / ZT_CW, g.sx2 - g.sx2 / 2 + 1);
     k_ztable<<<grid, 256, sm, st>>>(g, fg, zspec_table_stride(g), planes, 1.0 / (g.sx1 * g.dx1),
