@@ -90,7 +90,6 @@ __device__ __forceinline__ void pdl_enter() { pdl_wait(); }
 __device__ __forceinline__ float4 ld4(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
 __device__ __forceinline__ float4 ldc4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 __device__ __forceinline__ void st4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
-__device__ __forceinline__ float geti(const float4 &v, int j) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; }
 
 // 1/x by the hardware's approximate reciprocal (PTX rcp.approx.ftz.f32,
 // relative error about 2^-23; a subnormal x flushes to zero).  The x3

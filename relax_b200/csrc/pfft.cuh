@@ -76,9 +76,6 @@ __device__ __forceinline__ P pmul(P a, W w)
     return {fma2(neg2(a.i), w.y, p), fma2(a.r, w.y, q)};
 }
 __device__ __forceinline__ W2 w2(float4 v) { return {make_float2(v.x, v.y), make_float2(v.z, v.w)}; }
-// shared-memory form of a pair
-__device__ __forceinline__ P2 p2(float4 v) { return {make_float2(v.x, v.y), make_float2(v.z, v.w)}; }
-__device__ __forceinline__ float4 f4(P2 v) { return make_float4(v.r.x, v.r.y, v.i.x, v.i.y); }
 // two complex values of neighbouring lines that are neighbours in memory
 __device__ __forceinline__ P2 pair(float4 v) { return {make_float2(v.x, v.z), make_float2(v.y, v.w)}; }
 __device__ __forceinline__ float4 unpair(P2 v) { return make_float4(v.r.x, v.i.x, v.r.y, v.i.y); }

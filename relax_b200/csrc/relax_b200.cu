@@ -510,7 +510,7 @@ struct Spectral {
         cudaError_t re0 = cudaSuccess;
         if (use_reg) {
             TIMED(prof, ST_XFWD, st, (xr0 = xfwd_reg(xa, div, st, &re0)));
-            if (re0 != cudaSuccess) return fail(RELAX_ERR_CUDA, "k_xfwd_reg: %s", cudaGetErrorString(re0));
+            if (re0 != cudaSuccess) return fail(RELAX_ERR_CUDA, "xfwd_reg: %s", cudaGetErrorString(re0));
         }
         if (!xr0) {
             if (div) TIMED(prof, ST_XFWD, st, (k_xfwd<XIN_DIV><<<gx, RELAX_NTHREADS, smx, st>>>(xa)));
@@ -520,7 +520,7 @@ struct Spectral {
         cudaError_t re = cudaSuccess;
         if (use_reg) {
             TIMED(prof, ST_YFWD, st, (yreg = ypass_reg(ya, -1, st, &re)));
-            if (re != cudaSuccess) return fail(RELAX_ERR_CUDA, "k_ypass_reg: %s", cudaGetErrorString(re));
+            if (re != cudaSuccess) return fail(RELAX_ERR_CUDA, "ypass_reg: %s", cudaGetErrorString(re));
         }
         if (!use_reg || !yreg) {
             TIMED(prof, ST_YFWD, st,
@@ -535,7 +535,7 @@ struct Spectral {
         }
         if (use_reg && fg && !zr) {
             TIMED(prof, ST_ZSPEC, st, (zr = zspec_reg(za, st, &re)));
-            if (re != cudaSuccess) return fail(RELAX_ERR_CUDA, "k_zspec_reg: %s", cudaGetErrorString(re));
+            if (re != cudaSuccess) return fail(RELAX_ERR_CUDA, "zspec_reg: %s", cudaGetErrorString(re));
         }
         if (!zr) {
             za.tw = twz;
@@ -545,7 +545,7 @@ struct Spectral {
         bool yr2 = false;
         if (use_reg) {
             TIMED(prof, ST_YINV, st, (yr2 = ypass_reg(yb, +1, st, &re)));
-            if (re != cudaSuccess) return fail(RELAX_ERR_CUDA, "k_ypass_reg: %s", cudaGetErrorString(re));
+            if (re != cudaSuccess) return fail(RELAX_ERR_CUDA, "ypass_reg: %s", cudaGetErrorString(re));
         }
         if (!yr2) {
             TIMED(prof, ST_YINV, st,
@@ -556,7 +556,7 @@ struct Spectral {
         bool xr = false;
         if (use_reg) {
             TIMED(prof, ST_XINV, st, (xr = xinv_reg(xi, st, &re)));
-            if (re != cudaSuccess) return fail(RELAX_ERR_CUDA, "k_xinv_reg: %s", cudaGetErrorString(re));
+            if (re != cudaSuccess) return fail(RELAX_ERR_CUDA, "xinv_reg: %s", cudaGetErrorString(re));
         }
         if (!xr) TIMED(prof, ST_XINV, st, (k_xinv<<<dim3(g.sx2 / rows, nout), RELAX_NTHREADS, smx, st>>>(xi)));
         return RELAX_OK;

@@ -3,7 +3,7 @@
 // surfacetractioncowling, cerrutimodified and the inverse transform) with
 // its DFT sub-transforms on the 5th-generation tensor cores (tcgen05).
 //
-// Mixed-precision form of k_zspec_sm for a 128-deep FFT box and the step's
+// Mixed-precision form of the x3 pass (k_zpass) for a 128-deep FFT box and the step's
 // pruned transform (input planes [0, 64) non-zero, output planes [0, 64)
 // wanted).  A column of 128 points splits into two interleaved length-64
 // DFTs:
@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(ZT_THREADS, 1) k_zspec_tc(const __grid_constan
         }
         __syncthreads();
         // per-column FP64 combination (fixed order), surface traction, and the
-        // Cerruti coefficients of k_zspec_sm (src/green.f90:356-366, :578-609)
+        // Cerruti coefficients, as in k_zpass (src/green.f90:356-366, :578-609)
         if (tid < 64) {
             const int c = tid;
             float cc[14];
