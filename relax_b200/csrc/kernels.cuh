@@ -644,10 +644,11 @@ __global__ void __launch_bounds__(RELAX_NTHREADS, TRANS ? 2 : 3) k_stress(const 
 // Tiles of 128 groups and 4 blocks measured 710 us on the large box, the
 // strain ahead of the wait 96 us on the first, and the CORR pass in this form
 // 81 us against 71 (its stencil loads, not tau and m, are what it waits for).
+// TRANS, whose own state comes by plain loads: 47.7 -> 44.8 us on 128^3.
 constexpr int SP_STAGES = 2, SP_BLOCKS = 2, SP_TILE = RELAX_NTHREADS;
 constexpr size_t SP_SMEM = (size_t)SP_STAGES * 12 * SP_TILE * sizeof(float4);
 
-template <bool BATCH = false>
+template <bool BATCH, bool TRANS>
 __global__ void __launch_bounds__(SP_TILE, SP_BLOCKS) k_stress_pipe(const __grid_constant__ StressArgs a0)
 {
     pdl_enter();
@@ -699,7 +700,7 @@ __global__ void __launch_bounds__(SP_TILE, SP_BLOCKS) k_stress_pipe(const __grid
             return;
         }
         const size_t q = (size_t)tile * SP_TILE + threadIdx.x;
-        if (q < nq) stress_group<MODE_END, false, false>(a, q, src, tmin, amp_m, amp_t);
+        if (q < nq) stress_group<MODE_END, TRANS, false>(a, q, src, tmin, amp_m, amp_t);
         // The next tile into this one's place once every thread has used its
         // values (stored tau and m): a copy set off right after the reads can
         // overtake the reads that still wait in a warp's queue, which a
@@ -713,7 +714,7 @@ __global__ void __launch_bounds__(SP_TILE, SP_BLOCKS) k_stress_pipe(const __grid
             ph ^= 1;
         }
     }
-    stress_reduce<MODE_END, false>(a, tmin, amp_m, amp_t);
+    stress_reduce<MODE_END, TRANS>(a, tmin, amp_m, amp_t);
 }
 
 // tau += Dt m with the amplitude of m (coseismic-event path of the step,

@@ -1130,10 +1130,11 @@ static StressArgs stress_args(relax_ctx *c, const float *w)
 constexpr int kPipeBlocks = 148 * SP_BLOCKS;
 static bool pipe_ok(const Grid &g) { return (int)nblocks(g.nh / 4, SP_TILE) >= 2 * kPipeBlocks; }
 template <bool BATCH>
-static void launch_stress_pipe(const StressArgs &a, int nm, cudaStream_t st)
+static void launch_stress_pipe(const StressArgs &a, bool trans, int nm, cudaStream_t st)
 {
-    set_smem(k_stress_pipe<BATCH>, SP_SMEM);
-    launch_pdl(k_stress_pipe<BATCH>, dim3(kPipeBlocks, nm), SP_TILE, SP_SMEM, st, a);
+    auto k = trans ? k_stress_pipe<BATCH, true> : k_stress_pipe<BATCH, false>;
+    set_smem(k, SP_SMEM);
+    launch_pdl(k, dim3(kPipeBlocks, nm), SP_TILE, SP_SMEM, st, a);
 }
 
 template <int MODE>
@@ -1161,10 +1162,10 @@ static int launch_stress(relax_ctx *c, StressArgs a)
         TIMED(&c->prof, stage, c->st, (launch_pdl(k_stress<MODE, false, false, true>, c->nblk, RELAX_NTHREADS, 0, c->st, a)));
         return RELAX_OK;
     }
-    if (trans)
+    if (MODE == MODE_END && pipe_ok(c->g))
+        TIMED(&c->prof, stage, c->st, (launch_stress_pipe<false>(a, trans, 1, c->st)));
+    else if (trans)
         TIMED(&c->prof, stage, c->st, (launch_pdl(k_stress<MODE, false, true>, c->nblk, RELAX_NTHREADS, 0, c->st, a)));
-    else if (MODE == MODE_END && pipe_ok(c->g))
-        TIMED(&c->prof, stage, c->st, (launch_stress_pipe<false>(a, 1, c->st)));
     else
         TIMED(&c->prof, stage, c->st, (launch_pdl(k_stress<MODE>, c->nblk, RELAX_NTHREADS, 0, c->st, a)));
     return RELAX_OK;
@@ -3643,8 +3644,8 @@ static int batch_kernels(relax_batch *b)
     }
     CKL();
     TRY(batch_green(b, t.xic0));
-    if (b->trans) launch_pdl(k_stress<MODE_END, true, true>, dim3(c0->nblk, n), RELAX_NTHREADS, 0, st, t.end0);
-    else if (pipe_ok(c0->g)) launch_stress_pipe<true>(t.end0, n, st);
+    if (pipe_ok(c0->g)) launch_stress_pipe<true>(t.end0, b->trans, n, st);
+    else if (b->trans) launch_pdl(k_stress<MODE_END, true, true>, dim3(c0->nblk, n), RELAX_NTHREADS, 0, st, t.end0);
     else launch_pdl(k_stress<MODE_END, true>, dim3(c0->nblk, n), RELAX_NTHREADS, 0, st, t.end0);
     b->launches++;
     CKL();
